@@ -48,6 +48,10 @@ constexpr uint32_t kHashZ = 440817757u;
 // Particles per tile: one warp. Tiles never straddle scenes.
 constexpr int kTile = 32;
 
+// Neighbour-list entries per particle (pairs with dist <= r); a particle with
+// more neighbours is handled by the walk of its cells in the force passes.
+constexpr uint32_t kNbrCap = 64;
+
 // Per-scene descriptor, built on the host from sph_params.
 struct SceneDev {
   uint32_t n;         // particles
@@ -67,6 +71,7 @@ struct SceneDev {
   float cut_lo;       // cut_lt narrowed by 2e-6: an FMA estimate below it
                       // certifies d2 <= cut_lt without the exact recompute
   float r2;           // r*r
+  float inv_r;        // 1/r
   float vol2, vol3;   // density kernel scales   (kernels.h:28,40)
   float ds2h, ds3h;   // 0.5 * derivative scales (kernels.h:52,64)
   float vscale;       // poly6 scale             (kernels.h:76)

@@ -95,7 +95,9 @@ SceneDev MakeSceneDev(const sph_params& p, uint32_t n, uint32_t base, uint32_t t
   d.cut_lt = std::min(p.cutoff_sq, t_lt);
   d.cut_le = std::min(p.cutoff_sq, t_le);
   d.cut_hi = d.cut_le * 1.000002f;
-  d.cut_lo = d.cut_lt * 0.999998f;  d.r2 = r * r;
+  d.cut_lo = d.cut_lt * 0.999998f;
+  d.r2 = r * r;
+  d.inv_r = 1.0f / r;
   // kernels.h:28,40,52,64,76 -- same float expressions.
   d.vol2 = 15.0f / (2.0f * kPiF * powf(r, 5.0f));
   d.vol3 = 15.0f / (kPiF * powf(r, 6.0f));
@@ -209,7 +211,7 @@ int Engine::Init() {
   chk(Alloc(&ctx_.ncount, C));
   chk(Alloc(&ctx_.cell_first, C));
   chk(Alloc(&ctx_.cell_tab, C * 27ull));
-  chk(Alloc(&ctx_.nbr, C * static_cast<uint64_t>(kNbrCap)));
+  chk(Alloc(&ctx_.nbr, (C + 31) / 32 * 32 * kNbrCap));  // lists come in groups of 32 slots
   const uint64_t T = kTablePerParticle * C + kTableAllowance;  // key-table entries
   chk(Alloc(&ctx_.count, T));
   chk(Alloc(&ctx_.start, T + 1));
@@ -229,8 +231,6 @@ int Engine::Init() {
   ctx_.scenes = d_scenes_;
   ctx_.out4 = d_out4_;
   ctx_.status = d_status_;
-  ctx_.nbr_stride = static_cast<uint32_t>(C);
-  ctx_.nbr_cap = kNbrCap;
   return SPH_OK;
 }
 

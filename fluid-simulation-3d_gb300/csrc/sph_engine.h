@@ -165,9 +165,6 @@ class Engine {
   uint32_t* d_rcolour_ = nullptr;
   uint64_t render_pixels_ = 0;
 
-  // Neighbour-list capacity per particle (pairs with dist <= r); a particle
-  // with more neighbours is handled by the bucket walk in the force passes.
-  static constexpr uint32_t kNbrCap = 64;
   sph_tuning tuning_{128, 1, 32, 2, 0, 0};
   int sm_count_ = 0;
 

@@ -60,10 +60,8 @@ struct LaunchCtx {
   uint32_t* count = nullptr;
   uint32_t* start = nullptr;
   uint32_t* partial = nullptr;
-  uint32_t* nbr = nullptr;      // neighbour lists, nbr[k * nbr_stride + slot]
-  uint32_t* ncount = nullptr;   // neighbours per slot (> nbr_cap: overflow)
-  uint32_t nbr_stride = 0;
-  uint32_t nbr_cap = 0;
+  uint32_t* nbr = nullptr;      // neighbour lists, 64 entries a slot (nbr_index)
+  uint32_t* ncount = nullptr;   // neighbours per slot (> kNbrCap: overflow)
   int gather = 2;               // neighbour entries gathered per batch (2, 3, 4, 8)
   int lanes = 1;                // lanes per particle in the force kernels (1 or 2:
                                 // 32 or 16 particles per warp)
