@@ -50,14 +50,10 @@ __device__ __forceinline__ float dist2(float dx, float dy, float dz) {
 __device__ __forceinline__ float dist2_fast(float dx, float dy, float dz) {
   return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
 }
-// Hardware square root estimate (0 -> 0). Flushing denormals saves the walk
-// the range test and the two scalings of the plain form (172 -> 164 us at 1M,
-// 1204 -> 1140 us at 8.4M) and changes no density: the result is only used as
-// r - sqrt(d2), a denormal d2 has sqrt(d2) < 1.1e-19, and r - 1.1e-19 rounds
-// to r for every radius whose 1/r^5 kernel scale is finite.
+// Hardware square root estimate (sqrt.approx.f32: 0 -> 0).
 __device__ __forceinline__ float sqrt_approx(float x) {
   float y;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 
@@ -565,16 +561,12 @@ k_cell_table(const uint2* __restrict__ tiles, uint32_t ntiles,
 // reference's exact d2 (dropping the rare band pairs) and accumulates the
 // kernels; contributions vanish at the cutoff ((r-dist)^2), so the hardware
 // square root serves the kernel value. The self pair contributes (r, r).
-// One pair's share of the density sums, w = r - dist.
-__device__ __forceinline__ void density_sum(float w, float& s2, float& s3) {
+__device__ __forceinline__ void density_pair(const SceneDev& S, float d2,
+                                             float& s2, float& s3) {
+  const float w = S.r - sqrt_approx(d2);
   const float w2 = w * w;
   s2 += w2;
   s3 = fmaf(w2, w, s3);
-}
-
-__device__ __forceinline__ void density_pair(const SceneDev& S, float d2,
-                                             float& s2, float& s3) {
-  density_sum(S.r - sqrt_approx(d2), s2, s3);
 }
 
 __device__ __forceinline__ void density_store(const SceneDev& S, uint32_t i,
@@ -646,146 +638,13 @@ __global__ void __maxnreg__(32) k_density_walk(const uint2* __restrict__ tiles,
           wp += nbr_step;
         }
         ++cnt;
-        density_sum(r - sqrt_approx(d2), s2, s3);
+        const float w = r - sqrt_approx(d2);
+        const float w2 = w * w;
+        s2 += w2;
+        s3 = fmaf(w2, w, s3);
       }
     });
     density_store(S, i, s2, s3, cnt, dens_a, dens_b, ncount);
-  }
-}
-
-// Latency form for small launches: a warp takes eight slots. Lanes hold the
-// candidates of the eight particles' common neighbourhood (up to 256 at a time) in
-// registers; every particle is tested against all of them at once, a ballot
-// ranks the hits in candidate order, and r - dist of each goes to its rank in
-// shared memory, where one lane a particle sums them in that order. The list
-// and the sums are therefore those of k_density_walk bit for bit, but the
-// chain a particle waits for is four dependent loads and some 25 additions
-// instead of ~140 candidates one after another.
-constexpr int kCoopPer = 8;                          // particles a warp
-constexpr int kCoopSub = kTile / kCoopPer;           // warps a tile
-constexpr int kCoopBlock = 128;
-constexpr int kCoopWarps = kCoopBlock / 32;
-constexpr int kCoopChunks = 8;
-constexpr int kCoopRow = kCoopChunks * 32 + 1;       // odd: lanes read their rows without conflicts
-
-template <int kTables>
-__global__ void __launch_bounds__(kCoopBlock)
-k_density_coop(const uint2* __restrict__ tiles, uint32_t ntiles,
-               const SceneDev* __restrict__ scenes, const float4* __restrict__ pred,
-               const uint32_t* __restrict__ start, const uint32_t* __restrict__ cell_first,
-               const uint2* __restrict__ cell_tab, float2* __restrict__ dens_a,
-               float4* __restrict__ dens_b, uint32_t* __restrict__ nbr,
-               uint32_t* __restrict__ ncount) {
-  __shared__ float s_w[kCoopWarps][kCoopPer][kCoopRow];
-  pdl_enter();
-  const uint32_t lane = lane_id();
-  const uint32_t lt_mask = (1u << lane) - 1u;
-  float (*const sw)[kCoopRow] = s_w[threadIdx.x >> 5];
-  for (uint32_t v = warp_id_global(); v < ntiles * kCoopSub; v += warps_total()) {
-    const uint2 tile = tiles[v / kCoopSub];
-    const uint32_t sub = v % kCoopSub * kCoopPer, len = tile_len(tile);
-    if (sub >= len) continue;
-    const uint32_t m = min(len - sub, static_cast<uint32_t>(kCoopPer));
-    const SceneDev& S = scenes[tile_scene(tile)];
-    const bool direct = kTables == kTablesDirect    ? true
-                      : kTables == kTablesBuckets ? false
-                                                  : S.direct != 0u;
-    const uint32_t i0 = tile.y + sub;
-    const uint32_t i = i0 + min(lane, m - 1u);  // lanes 0..m-1 own a particle
-    const float4 me = pred[i];
-    const uint32_t cell = __float_as_uint(me.w);
-    const uint32_t cf = kTables == kTablesDirect ? 0u : cell_first[i];
-    const float cut = S.cut_le, r = S.r;
-    float s2 = S.r2, s3 = S.r2 * r;  // self: w = r
-    uint32_t cnt = 0;
-    uint32_t todo = (1u << m) - 1u;
-    while (todo) {
-      // the next particles that share one set of runs: a span of cells whose
-      // nine rows stay apart (grid table), one cell (bucket table)
-      const int lead = __ffs(todo) - 1;
-      const uint32_t c0 = __shfl_sync(kFull, cell, lead);
-      const uint32_t cf0 = __shfl_sync(kFull, cf, lead);
-      const bool in = lane < m && ((todo >> lane) & 1u) &&
-                      (direct ? cell - c0 + 3u <= S.gwy : cf == cf0);
-      const uint32_t gm = __ballot_sync(kFull, in);
-      todo &= ~gm;
-      const int last = 31 - __clz(gm);
-      uint2 run = make_uint2(0u, 0u);
-      if (direct) {
-        const uint32_t cN = __shfl_sync(kFull, cell, last);
-        if (lane < 9u) {
-          const uint32_t off = S.tbase + (lane / 3u - 1u) * S.gwy + (lane % 3u - 1u) * S.gwz;
-          run.x = __ldg(start + (c0 + off - 1u));
-          run.y = __ldg(start + (cN + off + 2u)) - run.x;
-        }
-      } else {
-        if (lane < 27u) run = __ldg(cell_tab + static_cast<uint64_t>(cf0) * 27u + lane);
-        // a merged row keeps its run in its first entry; the other two are unused
-        const uint32_t heads =
-            __ballot_sync(kFull, lane < 27u && lane % 3u == 0u && (run.y & kRunMerged));
-        if (lane % 3u != 0u && ((heads >> (lane - lane % 3u)) & 1u)) run.y = 0u;
-        run.y &= ~kRunMerged;
-      }
-      const uint32_t incl = warp_incl_scan(run.y);
-      const uint32_t excl = incl - run.y;
-      const uint32_t total = __shfl_sync(kFull, incl, 31);
-      for (uint32_t seg = 0; seg < total; seg += kCoopChunks * 32u) {
-        float4 q[kCoopChunks];
-        uint32_t js[kCoopChunks];
-#pragma unroll
-        for (int c = 0; c < kCoopChunks; ++c) {
-          const uint32_t e = seg + c * 32u + lane;
-          // o = number of runs ending at or before e (incl is ascending)
-          uint32_t o = 0;
-#pragma unroll
-          for (uint32_t step = 16; step >= 1; step >>= 1) {
-            const uint32_t probe = o + step - 1u;
-            const uint32_t x = __shfl_sync(kFull, incl, probe & 31u);
-            if (probe < 27u && x <= e) o += step;
-          }
-          const uint32_t src = min(o, 26u);
-          js[c] = __shfl_sync(kFull, run.x, src) + (e - __shfl_sync(kFull, excl, src));
-          q[c] = e < total ? __ldg(pred + js[c])
-                           : make_float4(__int_as_float(0x7f800000), 0.f, 0.f, 0.f);
-        }
-        uint32_t hits = 0;  // of this lane's particle in this segment
-        for (int pp = lead; pp <= last; ++pp) {
-          const float2 npxy =
-              make_float2(-__shfl_sync(kFull, me.x, pp), -__shfl_sync(kFull, me.y, pp));
-          const float pz = __shfl_sync(kFull, me.z, pp);
-          const uint32_t before = __shfl_sync(kFull, cnt, pp);
-          const uint32_t ip = i0 + static_cast<uint32_t>(pp);
-          uint32_t* const list = nbr + nbr_index(ip, 0);
-          uint32_t base = 0;
-#pragma unroll
-          for (int c = 0; c < kCoopChunks; ++c) {
-            if (seg + c * 32u >= total) break;
-            const float2 dxy = __fadd2_rn(make_float2(q[c].x, q[c].y), npxy);
-            const float2 sxy = __fmul2_rn(dxy, dxy);
-            const float dz = q[c].z - pz;
-            const float d2 = __fadd_rn(__fadd_rn(sxy.x, sxy.y), __fmul_rn(dz, dz));
-            const bool hit = d2 <= cut && js[c] != ip;
-            const uint32_t hm = __ballot_sync(kFull, hit);
-            if (hit) {
-              const uint32_t k = base + __popc(hm & lt_mask);
-              sw[pp][k] = r - sqrt_approx(d2);
-              if (before + k < kNbrCap) list[(before + k) * 32u] = js[c];
-            }
-            base += __popc(hm);
-          }
-          if (lane == static_cast<uint32_t>(pp)) hits = base;
-        }
-        __syncwarp();
-        if (lane < kCoopPer) {
-          const float* row = sw[lane];
-#pragma unroll 4
-          for (uint32_t k = 0; k < hits; ++k) density_sum(row[k], s2, s3);
-        }
-        cnt += hits;
-        __syncwarp();  // the next segment rewrites the rows
-      }
-    }
-    if (lane < m) density_store(S, i, s2, s3, cnt, dens_a, dens_b, ncount);
   }
 }
 
@@ -923,21 +782,16 @@ __global__ void k_density(const uint2* __restrict__ tiles, uint32_t ntiles,
 // entries at a time so their neighbours' gathers are in flight together, the
 // next batch's entries loading meanwhile. A list that overflowed
 // falls back to the walk of the cell's runs.
-__device__ __forceinline__ float pressure_term(const SceneDev& S, float d2, float Pi, float Pni,
-                                               float4 b) {
-  const float dist = __fsqrt_rn(d2);
-  const float w = S.r - dist;
-  const float a2 = S.ds2h * fmaf(Pi, b.x, b.y);
-  const float a3 = S.ds3h * w * fmaf(Pni, b.z, b.w);
-  return -w * (a2 + a3);
-}
-
 __device__ __forceinline__ void pressure_pair(const SceneDev& S, float3 p,
                                               float Pi, float Pni, float4 q,
                                               float4 b, float3& f) {
   const float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
   const float d2 = dist2(dx, dy, dz);
-  const float tsum = pressure_term(S, d2, Pi, Pni, b);
+  const float dist = __fsqrt_rn(d2);
+  const float w = S.r - dist;
+  const float a2 = S.ds2h * fmaf(Pi, b.x, b.y);
+  const float a3 = S.ds3h * w * fmaf(Pni, b.z, b.w);
+  const float tsum = -w * (a2 + a3);
   if (d2 > 0.0f) {
     const float s = tsum * rsqrtf(d2);
     f.x = fmaf(dx, s, f.x);
@@ -947,6 +801,8 @@ __device__ __forceinline__ void pressure_pair(const SceneDev& S, float3 p,
     f.y += tsum;  // dir = (0,1,0) for coincident particles (:414)
   }
 }
+
+
 
 // kLanes lanes per particle (tuning.particles_per_warp = 32 / kLanes): a
 // warp takes its tile's 32 particles in kLanes passes of 32 / kLanes; lane
@@ -1033,97 +889,6 @@ __global__ void k_pressure(const uint2* __restrict__ tiles, uint32_t ntiles,
   }
 }
 
-// Latency form for small launches, as k_density_coop: eight particles a warp,
-// four lanes a particle evaluate every fourth list entry each and leave (direction,
-// magnitude) in shared memory; one lane a component sums them in list order,
-// with the operations of pressure_pair, so the result is k_pressure's bit for bit.
-constexpr int kCoopTerms = kNbrCap + 1;  // float4 rows, shifted a bank group each
-constexpr int kCoopGather = 4;           // entries a lane has in flight
-
-// Component `comp` of the ordered sum of fma(direction, magnitude) over a row.
-__device__ __forceinline__ float coop_sum(const float4* row, uint32_t comp, uint32_t cnt) {
-  const float* p = reinterpret_cast<const float*>(row);
-  float f = 0.0f;
-#pragma unroll 4
-  for (uint32_t k = 0; k < cnt; ++k) f = fmaf(p[4u * k + comp], p[4u * k + 3u], f);
-  return f;
-}
-
-template <int kTables>
-__global__ void __launch_bounds__(kCoopBlock)
-k_pressure_coop(const uint2* __restrict__ tiles, uint32_t ntiles,
-                const SceneDev* __restrict__ scenes, const float4* __restrict__ pred,
-                const uint32_t* __restrict__ start, const uint32_t* __restrict__ cell_first,
-                const uint2* __restrict__ cell_tab, const float2* __restrict__ dens_a,
-                const float4* __restrict__ dens_b, const uint32_t* __restrict__ nbr,
-                const uint32_t* __restrict__ ncount, const float4* __restrict__ vel,
-                float4* __restrict__ rec_v, float4* __restrict__ dbg_accp) {
-  __shared__ float4 s_t[kCoopWarps][kCoopPer][kCoopTerms];
-  pdl_enter();
-  const uint32_t lane = lane_id();
-  const uint32_t pp = lane % kCoopPer, part = lane / kCoopPer;
-  float4* const row = s_t[threadIdx.x >> 5][pp];
-  for (uint32_t v = warp_id_global(); v < ntiles * kCoopSub; v += warps_total()) {
-    const uint2 tile = tiles[v / kCoopSub];
-    const uint32_t sub = v % kCoopSub * kCoopPer, len = tile_len(tile);
-    if (sub >= len) continue;
-    const SceneDev& S = scenes[tile_scene(tile)];
-    const bool live = sub + pp < len;
-    const uint32_t i = tile.y + min(sub + pp, len - 1u);
-    const float4 pi = pred[i];
-    const float3 p = make_float3(pi.x, pi.y, pi.z);
-    const float2 di = dens_a[i];
-    const float4 vi = vel[i];
-    const float Pi = (di.x - S.rho0) * S.k, Pni = di.y * S.kn;
-    const uint32_t cnt = live ? ncount[i] : 0u;
-    float3 f = make_float3(0.0f, 0.0f, 0.0f);
-    if (cnt <= kNbrCap) {
-      for (uint32_t k0 = part; k0 < cnt; k0 += 4u * kCoopGather) {
-        uint32_t j[kCoopGather];
-        float4 q[kCoopGather], b[kCoopGather];
-        load_nbr_batch<kCoopGather, 4>(nbr, i, k0, cnt, j);
-#pragma unroll
-        for (int u = 0; u < kCoopGather; ++u) {
-          if (k0 + 4u * u < cnt) {
-            q[u] = __ldg(pred + j[u]);
-            b[u] = __ldg(dens_b + j[u]);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kCoopGather; ++u) {
-          if (k0 + 4u * u < cnt) {
-            const float dx = q[u].x - p.x, dy = q[u].y - p.y, dz = q[u].z - p.z;
-            const float d2 = dist2(dx, dy, dz);
-            const float tsum = pressure_term(S, d2, Pi, Pni, b[u]);
-            row[k0 + 4u * u] = d2 > 0.0f ? make_float4(dx, dy, dz, tsum * rsqrtf(d2))
-                                         : make_float4(0.0f, 1.0f, 0.0f, tsum);
-          }
-        }
-      }
-    } else if (part == 0) {
-      walk_runs<kTables>(S, start, cell_tab, cell_first[i], __float_as_uint(pi.w), pred,
-                         [&](uint32_t j, float4 q) {
-        if (j == i) return;
-        const float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
-        if (dist2(dx, dy, dz) <= S.cut_le)
-          pressure_pair(S, p, Pi, Pni, q, __ldg(dens_b + j), f);
-      });
-    }
-    __syncwarp();
-    const float fc = coop_sum(row, min(part, 2u), cnt <= kNbrCap ? cnt : 0u);
-    const float fx = __shfl_sync(kFull, fc, pp), fy = __shfl_sync(kFull, fc, kCoopPer + pp),
-                fz = __shfl_sync(kFull, fc, 2 * kCoopPer + pp);
-    if (cnt <= kNbrCap) f = make_float3(fx, fy, fz);
-    __syncwarp();  // the next slots rewrite the rows
-    if (!live || part != 0) continue;
-    const float inv_rho = 1.0f / di.x;
-    const float ax = f.x * inv_rho, ay = f.y * inv_rho, az = f.z * inv_rho;
-    store_rec(rec_v, i, pi,
-              make_float4(vi.x + ax * S.dt, vi.y + ay * S.dt, vi.z + az * S.dt, 0.f));
-    if (dbg_accp) dbg_accp[i] = make_float4(ax, ay, az, 0.0f);
-  }
-}
-
 // ------------------------------------------------ viscosity + integrate
 // CalculateViscosityForce (:424-464) over the neighbour list reading the
 // post-pressure snapshot (Jacobi); poly6 = (r^2 - d^2)^3 for dist < r. Then
@@ -1142,39 +907,6 @@ __device__ __forceinline__ void visc_pair(const SceneDev& S, float3 p,
     f.y = fmaf(vj.y - vi.y, w3, f.y);
     f.z = fmaf(vj.z - vi.z, w3, f.z);
   }
-}
-
-// The viscosity increment f of slot i, then the integration and the box
-// collision; with fuse_next also the key of the new state's prediction (S_next
-// is the same scene: its grid constants are read there, not kept in registers
-// through the sum).
-__device__ __forceinline__ void integrate(const SceneDev& S, const SceneDev& S_next, uint32_t i,
-                                          float4 vi, float3 f, float4* __restrict__ pos,
-                                          float4* __restrict__ vel, float4* __restrict__ out4,
-                                          int fuse_next, float4* __restrict__ dbg_velv,
-                                          uint32_t& key, uint32_t& cell, uint32_t& id, bool& bad) {
-  const float c = S.vscale * S.mu * S.dt;
-  float3 v = make_float3(vi.x + f.x * c, vi.y + f.y * c, vi.z + f.z * c);
-  if (dbg_velv) dbg_velv[i] = make_float4(v.x, v.y, v.z, 0.0f);
-  float4 x = pos[i];
-  x.x = __fadd_rn(x.x, __fmul_rn(v.x, S.dt));
-  x.y = __fadd_rn(x.y, __fmul_rn(v.y, S.dt));
-  x.z = __fadd_rn(x.z, __fmul_rn(v.z, S.dt));
-  // edgeDst = halfSize - |pos|; if <= 0 clamp to the wall and reflect.
-  if (S.hx - fabsf(x.x) <= 0.0f) { x.x = S.hx * copysign_or_zero(x.x); v.x *= S.ndamp; }
-  if (S.hy - fabsf(x.y) <= 0.0f) { x.y = S.hy * copysign_or_zero(x.y); v.y *= S.ndamp; }
-  if (S.hz - fabsf(x.z) <= 0.0f) { x.z = S.hz * copysign_or_zero(x.z); v.z *= S.ndamp; }
-  pos[i] = x;
-  const float4 v4 = make_float4(v.x, v.y, v.z, 0.0f);
-  vel[i] = v4;
-  bad = !(isfinite(x.x) && isfinite(x.y) && isfinite(x.z) &&
-          isfinite(v.x) && isfinite(v.y) && isfinite(v.z));
-  id = __float_as_uint(x.w);
-  if (out4) {
-    if (id < S.n) out4[S.base + id] = make_float4(x.x, x.y, x.z, 0.34f);
-    else bad = true;
-  }
-  if (fuse_next) predict_key(S_next, x, v4, key, cell);
 }
 
 // kLanes lanes per particle as in k_pressure.
@@ -1240,8 +972,29 @@ __global__ void k_visc_integrate(
         f.z += __shfl_xor_sync(kFull, f.z, 16);
       }
       if (live) {
-        integrate(S, scenes[tile_scene(tile)], i, vi, f, pos, vel, out4, fuse_next, dbg_velv, key,
-                  cell, id, bad);
+        const float c = S.vscale * S.mu * S.dt;
+        float3 v = make_float3(vi.x + f.x * c, vi.y + f.y * c, vi.z + f.z * c);
+        if (dbg_velv) dbg_velv[i] = make_float4(v.x, v.y, v.z, 0.0f);
+        float4 x = pos[i];
+        x.x = __fadd_rn(x.x, __fmul_rn(v.x, S.dt));
+        x.y = __fadd_rn(x.y, __fmul_rn(v.y, S.dt));
+        x.z = __fadd_rn(x.z, __fmul_rn(v.z, S.dt));
+        // edgeDst = halfSize - |pos|; if <= 0 clamp to the wall and reflect.
+        if (S.hx - fabsf(x.x) <= 0.0f) { x.x = S.hx * copysign_or_zero(x.x); v.x *= S.ndamp; }
+        if (S.hy - fabsf(x.y) <= 0.0f) { x.y = S.hy * copysign_or_zero(x.y); v.y *= S.ndamp; }
+        if (S.hz - fabsf(x.z) <= 0.0f) { x.z = S.hz * copysign_or_zero(x.z); v.z *= S.ndamp; }
+        pos[i] = x;
+        const float4 v4 = make_float4(v.x, v.y, v.z, 0.0f);
+        vel[i] = v4;
+        bad = !(isfinite(x.x) && isfinite(x.y) && isfinite(x.z) &&
+                isfinite(v.x) && isfinite(v.y) && isfinite(v.z));
+        id = __float_as_uint(x.w);
+        if (out4) {
+          if (id < S.n) out4[S.base + id] = make_float4(x.x, x.y, x.z, 0.34f);
+          else bad = true;
+        }
+        // the grid constants are read here, not kept in registers through the loop
+        if (fuse_next) predict_key(scenes[tile_scene(tile)], x, v4, key, cell);
       }
       if (fuse_next) {
         const uint32_t r = aggregated_rank(count, key, live);
@@ -1249,79 +1002,6 @@ __global__ void k_visc_integrate(
       }
       if (__any_sync(kFull, bad) && lane == 0) flag(status, kStatusNonFinite);
     }
-  }
-}
-
-// Latency form for small launches, as k_pressure_coop: the terms of visc_pair
-// by four lanes a particle, summed in list order.
-template <int kTables>
-__global__ void __launch_bounds__(kCoopBlock) k_visc_coop(
-    const uint2* __restrict__ tiles, uint32_t ntiles, const SceneDev* __restrict__ scenes,
-    const float4* __restrict__ pred, const uint32_t* __restrict__ start,
-    const uint32_t* __restrict__ cell_first, const uint2* __restrict__ cell_tab,
-    const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ ncount,
-    const float4* __restrict__ rec_v, float4* __restrict__ pos, float4* __restrict__ vel,
-    float4* __restrict__ out4, int fuse_next, uint32_t* __restrict__ count,
-    uint4* __restrict__ keyrank, float4* __restrict__ dbg_velv, uint32_t* status) {
-  __shared__ float4 s_t[kCoopWarps][kCoopPer][kCoopTerms];
-  pdl_enter();
-  const uint32_t lane = lane_id();
-  const uint32_t pp = lane % kCoopPer, part = lane / kCoopPer;
-  float4* const row = s_t[threadIdx.x >> 5][pp];
-  for (uint32_t v = warp_id_global(); v < ntiles * kCoopSub; v += warps_total()) {
-    const uint2 tile = tiles[v / kCoopSub];
-    const uint32_t sub = v % kCoopSub * kCoopPer, len = tile_len(tile);
-    if (sub >= len) continue;
-    const SceneDev& S = scenes[tile_scene(tile)];
-    const bool in_tile = sub + pp < len;
-    const uint32_t i = tile.y + min(sub + pp, len - 1u);
-    float4 pi, vi;
-    load_rec(rec_v, i, pi, vi);
-    const float3 p = make_float3(pi.x, pi.y, pi.z);
-    const uint32_t cnt = in_tile ? ncount[i] : 0u;
-    float3 f = make_float3(0.0f, 0.0f, 0.0f);
-    if (cnt <= kNbrCap) {
-      for (uint32_t k0 = part; k0 < cnt; k0 += 4u * kCoopGather) {
-        uint32_t j[kCoopGather];
-        float4 q[kCoopGather], vj[kCoopGather];
-        load_nbr_batch<kCoopGather, 4>(nbr, i, k0, cnt, j);
-#pragma unroll
-        for (int u = 0; u < kCoopGather; ++u)
-          if (k0 + 4u * u < cnt) load_rec(rec_v, j[u], q[u], vj[u]);
-#pragma unroll
-        for (int u = 0; u < kCoopGather; ++u) {
-          if (k0 + 4u * u < cnt) {
-            const float dx = q[u].x - p.x, dy = q[u].y - p.y, dz = q[u].z - p.z;
-            const float d2 = dist2(dx, dy, dz);
-            const float w = S.r2 - d2;
-            row[k0 + 4u * u] = d2 <= S.cut_lt
-                                   ? make_float4(vj[u].x - vi.x, vj[u].y - vi.y, vj[u].z - vi.z,
-                                                 w * w * w)
-                                   : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          }
-        }
-      }
-    } else if (part == 0) {
-      walk_runs<kTables>(S, start, cell_tab, cell_first[i], __float_as_uint(pi.w), pred,
-                         [&](uint32_t j, float4 q) {
-        if (j != i) visc_pair(S, p, vi, q, __ldg(rec_v + 2ull * j + 1), f);
-      });
-    }
-    __syncwarp();
-    const float fc = coop_sum(row, min(part, 2u), cnt <= kNbrCap ? cnt : 0u);
-    const float fx = __shfl_sync(kFull, fc, pp), fy = __shfl_sync(kFull, fc, kCoopPer + pp),
-                fz = __shfl_sync(kFull, fc, 2 * kCoopPer + pp);
-    if (cnt <= kNbrCap) f = make_float3(fx, fy, fz);
-    __syncwarp();  // the next slots rewrite the rows
-    const bool live = in_tile && part == 0u;
-    bool bad = false;
-    uint32_t key = 0, cell = 0, id = 0;
-    if (live) integrate(S, S, i, vi, f, pos, vel, out4, fuse_next, dbg_velv, key, cell, id, bad);
-    if (fuse_next) {
-      const uint32_t r = aggregated_rank(count, key, live);
-      if (live) keyrank[i] = make_uint4(key, r, cell, id);
-    }
-    if (__any_sync(kFull, bad) && lane == 0) flag(status, kStatusNonFinite);
   }
 }
 
@@ -1702,21 +1382,9 @@ cudaError_t launch_sort_reorder(const LaunchCtx& c, const Tiles& old_tiles,
   return e;
 }
 
-// Whether a launch over `ntiles` tiles takes the latency forms.
-constexpr uint32_t kCoopTiles = 2048;
-bool coop_form(const LaunchCtx&, uint32_t ntiles) { return ntiles <= kCoopTiles; }
-
 cudaError_t launch_density(const LaunchCtx& c, const Tiles& tiles,
                            cudaStream_t st) {
   if (tiles.n == 0) return cudaSuccess;
-  if (coop_form(c, tiles.n) && c.cell_tile <= 1)
-    return launch_pdl(c.pdl,
-                      c.tables == kTablesDirect    ? k_density_coop<kTablesDirect>
-                      : c.tables == kTablesBuckets ? k_density_coop<kTablesBuckets>
-                                                   : k_density_coop<kTablesMixed>,
-                      grid_for(tiles.n * kCoopSub, kCoopBlock, c.max_blocks), kCoopBlock, st,
-                      tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab,
-                      c.dens_a, c.dens_b, c.nbr, c.ncount);
   const int b = c.block_nbr;
   const uint32_t g = grid_for(tiles.n, b, c.max_blocks);
   if (c.cell_tile <= 1)
@@ -1767,14 +1435,6 @@ auto visc_kernel(int gather, int lanes) {
 cudaError_t launch_pressure(const LaunchCtx& c, const Tiles& tiles,
                             cudaStream_t st) {
   if (tiles.n == 0) return cudaSuccess;
-  if (coop_form(c, tiles.n) && c.lanes == 1)
-    return launch_pdl(c.pdl,
-                      c.tables == kTablesDirect    ? k_pressure_coop<kTablesDirect>
-                      : c.tables == kTablesBuckets ? k_pressure_coop<kTablesBuckets>
-                                                   : k_pressure_coop<kTablesMixed>,
-                      grid_for(tiles.n * kCoopSub, kCoopBlock, c.max_blocks), kCoopBlock, st,
-                      tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab,
-                      c.dens_a, c.dens_b, c.nbr, c.ncount, c.vel2, c.rec_v, c.dbg_accp);
   const int b = c.block_force;
   auto kern = c.tables == kTablesDirect    ? pressure_kernel<kTablesDirect>(c.gather, c.lanes)
               : c.tables == kTablesBuckets ? pressure_kernel<kTablesBuckets>(c.gather, c.lanes)
@@ -1789,15 +1449,6 @@ cudaError_t launch_visc_integrate(const LaunchCtx& c, const Tiles& tiles,
                                   int fuse_next, int write_out,
                                   cudaStream_t st) {
   if (tiles.n == 0) return cudaSuccess;
-  if (coop_form(c, tiles.n) && c.lanes == 1)
-    return launch_pdl(c.pdl,
-                      c.tables == kTablesDirect    ? k_visc_coop<kTablesDirect>
-                      : c.tables == kTablesBuckets ? k_visc_coop<kTablesBuckets>
-                                                   : k_visc_coop<kTablesMixed>,
-                      grid_for(tiles.n * kCoopSub, kCoopBlock, c.max_blocks), kCoopBlock, st,
-                      tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab, c.nbr,
-                      c.ncount, c.rec_v, c.pos2, c.vel2, write_out ? c.out4 : nullptr, fuse_next,
-                      c.count, c.keyrank, c.dbg_velv, c.status);
   const int b = c.block_force;
   auto kern = c.tables == kTablesDirect    ? visc_kernel<kTablesDirect>(c.gather, c.lanes)
               : c.tables == kTablesBuckets ? visc_kernel<kTablesBuckets>(c.gather, c.lanes)
