@@ -50,10 +50,14 @@ __device__ __forceinline__ float dist2(float dx, float dy, float dz) {
 __device__ __forceinline__ float dist2_fast(float dx, float dy, float dz) {
   return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
 }
-// Hardware square root estimate (sqrt.approx.f32: 0 -> 0).
+// Hardware square root estimate (0 -> 0). Flushing denormals saves the walk
+// the range test and the two scalings of the plain form (172 -> 164 us at 1M,
+// 1204 -> 1140 us at 8.4M) and changes no density: the result is only used as
+// r - sqrt(d2), a denormal d2 has sqrt(d2) < 1.1e-19, and r - 1.1e-19 rounds
+// to r for every radius whose 1/r^5 kernel scale is finite.
 __device__ __forceinline__ float sqrt_approx(float x) {
   float y;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 
