@@ -565,12 +565,16 @@ k_cell_table(const uint2* __restrict__ tiles, uint32_t ntiles,
 // reference's exact d2 (dropping the rare band pairs) and accumulates the
 // kernels; contributions vanish at the cutoff ((r-dist)^2), so the hardware
 // square root serves the kernel value. The self pair contributes (r, r).
-__device__ __forceinline__ void density_pair(const SceneDev& S, float d2,
-                                             float& s2, float& s3) {
-  const float w = S.r - sqrt_approx(d2);
+// One pair's share of the density sums, w = r - dist.
+__device__ __forceinline__ void density_sum(float w, float& s2, float& s3) {
   const float w2 = w * w;
   s2 += w2;
   s3 = fmaf(w2, w, s3);
+}
+
+__device__ __forceinline__ void density_pair(const SceneDev& S, float d2,
+                                             float& s2, float& s3) {
+  density_sum(S.r - sqrt_approx(d2), s2, s3);
 }
 
 __device__ __forceinline__ void density_store(const SceneDev& S, uint32_t i,
@@ -642,15 +646,136 @@ __global__ void __maxnreg__(32) k_density_walk(const uint2* __restrict__ tiles,
           wp += nbr_step;
         }
         ++cnt;
-        const float w = r - sqrt_approx(d2);
-        const float w2 = w * w;
-        s2 += w2;
-        s3 = fmaf(w2, w, s3);
+        density_sum(r - sqrt_approx(d2), s2, s3);
       }
     });
     density_store(S, i, s2, s3, cnt, dens_a, dens_b, ncount);
   }
 }
+
+// Latency form for small launches (kRowsTiles): nine warps (a block) share a
+// tile, lane = particle, one row of the walk a warp. A pair within the cutoff
+// goes (distance squared, slot) to the lane's queue in shared memory; after a
+// barrier every warp moves its entries to their place in the particle's list --
+// rows in walk order, so the list is k_density_walk's -- and leaves r - dist
+// of each there for the first warp to sum in that order. The sums are therefore
+// the walk's bit for bit, while the chain a particle waits for is one row of
+// ~16 candidates instead of ~140 (measured: 16,384 particles 32 -> 11 us, 1,000
+// 39 -> 11 us). A particle with more hits than a queue or a list holds walks
+// all its rows again by itself. The 46 KB a block take the SM's occupancy, so
+// large launches lose (1M: 165 -> 292 us).
+constexpr int kRowWarps = 9;
+constexpr uint32_t kRowCap = 16;  // hits a queue holds
+
+template <int kTables>
+__global__ void __launch_bounds__(32 * kRowWarps)
+k_density_rows(const uint2* __restrict__ tiles, uint32_t ntiles,
+               const SceneDev* __restrict__ scenes, const float4* __restrict__ pred,
+               const uint32_t* __restrict__ start, const uint32_t* __restrict__ cell_first,
+               const uint2* __restrict__ cell_tab, float2* __restrict__ dens_a,
+               float4* __restrict__ dens_b, uint32_t* __restrict__ nbr,
+               uint32_t* __restrict__ ncount) {
+  __shared__ float2 s_hit[kRowWarps][kRowCap][32];
+  __shared__ float s_w[kNbrCap][32];
+  __shared__ uint32_t s_cnt[kRowWarps][32];
+  pdl_enter();
+  const uint32_t lane = lane_id(), s = threadIdx.x >> 5;
+  for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const uint2 tile = tiles[t];
+    const SceneDev& S = scenes[tile_scene(tile)];
+    const bool direct = kTables == kTablesDirect    ? true
+                      : kTables == kTablesBuckets ? false
+                                                  : S.direct != 0u;
+    const bool live = lane < tile_len(tile);
+    const uint32_t i = tile.y + (live ? lane : 0u);
+    const float4 me = pred[i];
+    const uint32_t cell = __float_as_uint(me.w);
+    const uint32_t cf = kTables == kTablesDirect ? 0u : cell_first[i];
+    const float cut = S.cut_le, r = S.r;
+    const float2 npxy = make_float2(-me.x, -me.y);
+    uint32_t cnt = 0;
+    auto run = [&](uint32_t j, uint32_t e) {
+      float4 next = __ldg(pred + (j < e ? j : i));
+      while (j < e) {
+        const float4 q = next;
+        next = __ldg(pred + (j + 1u < e ? j + 1u : j));  // the next candidate loads meanwhile
+        const float2 dxy = __fadd2_rn(make_float2(q.x, q.y), npxy);
+        const float2 sxy = __fmul2_rn(dxy, dxy);
+        const float dz = q.z - me.z;
+        const float d2 = __fadd_rn(__fadd_rn(sxy.x, sxy.y), __fmul_rn(dz, dz));
+        if (d2 <= cut && j != i) {
+          if (cnt < kRowCap) s_hit[s][cnt][lane] = make_float2(d2, __uint_as_float(j));
+          ++cnt;
+        }
+        ++j;
+      }
+    };
+    if (live) {
+      if (direct) {
+        const uint32_t k = S.tbase + cell + (s / 3u - 1u) * S.gwy + (s % 3u - 1u) * S.gwz;
+        run(__ldg(start + k - 1), __ldg(start + k + 2));
+      } else {
+        const uint2* tab = cell_tab + static_cast<uint64_t>(cf) * 27u + s * 3u;
+        const uint2 m = __ldg(tab);
+        if (m.y & kRunMerged) {
+          run(m.x, m.x + (m.y & ~kRunMerged));
+        } else {
+#pragma unroll 1
+          for (int k = 0; k < 3; ++k) {
+            const uint2 x = k ? __ldg(tab + k) : m;
+            run(x.x, x.x + x.y);
+          }
+        }
+      }
+    }
+    s_cnt[s][lane] = cnt;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+    bool full = false;
+#pragma unroll
+    for (uint32_t u = 0; u < kRowWarps; ++u) {
+      const uint32_t c = s_cnt[u][lane];
+      before += u < s ? c : 0u;
+      total += c;
+      full |= c > kRowCap;
+    }
+    full |= total > kNbrCap;
+    uint32_t* const list = nbr + nbr_index(i, 0);
+    if (!full) {
+      for (uint32_t k = 0; k < cnt; ++k) {
+        const float2 h = s_hit[s][k][lane];
+        s_w[before + k][lane] = r - sqrt_approx(h.x);
+        list[(before + k) * 32u] = __float_as_uint(h.y);
+      }
+    }
+    __syncthreads();
+    if (s == 0 && live) {
+      float s2 = S.r2, s3 = S.r2 * r;  // self: w = r
+      if (!full) {
+#pragma unroll 4
+        for (uint32_t k = 0; k < total; ++k) density_sum(s_w[k][lane], s2, s3);
+      } else {
+        uint32_t k = 0;
+        walk_runs<kTables>(S, start, cell_tab, cf, cell, pred, [&](uint32_t j, float4 q) {
+          const float d2 = dist2(q.x - me.x, q.y - me.y, q.z - me.z);
+          if (d2 <= cut && j != i) {
+            if (k < kNbrCap) list[k * 32u] = j;
+            ++k;
+            density_sum(r - sqrt_approx(d2), s2, s3);
+          }
+        });
+      }
+      density_store(S, i, s2, s3, total, dens_a, dens_b, ncount);
+    }
+    __syncthreads();  // the next tile rewrites the queues
+  }
+}
+
+// Eight particles a warp in the latency forms of the force kernels.
+constexpr int kCoopPer = 8;
+constexpr int kCoopSub = kTile / kCoopPer;  // warps a tile
+constexpr int kCoopBlock = 128;
+constexpr int kCoopWarps = kCoopBlock / 32;
 
 // Phase 1 is warp-cooperative over the cells of the warp's 32 slots: for
 // each cell, lanes 0..26 fetch its 27 runs, a warp scan gives their offsets
@@ -786,16 +911,21 @@ __global__ void k_density(const uint2* __restrict__ tiles, uint32_t ntiles,
 // entries at a time so their neighbours' gathers are in flight together, the
 // next batch's entries loading meanwhile. A list that overflowed
 // falls back to the walk of the cell's runs.
+__device__ __forceinline__ float pressure_term(const SceneDev& S, float d2, float Pi, float Pni,
+                                               float4 b) {
+  const float dist = __fsqrt_rn(d2);
+  const float w = S.r - dist;
+  const float a2 = S.ds2h * fmaf(Pi, b.x, b.y);
+  const float a3 = S.ds3h * w * fmaf(Pni, b.z, b.w);
+  return -w * (a2 + a3);
+}
+
 __device__ __forceinline__ void pressure_pair(const SceneDev& S, float3 p,
                                               float Pi, float Pni, float4 q,
                                               float4 b, float3& f) {
   const float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
   const float d2 = dist2(dx, dy, dz);
-  const float dist = __fsqrt_rn(d2);
-  const float w = S.r - dist;
-  const float a2 = S.ds2h * fmaf(Pi, b.x, b.y);
-  const float a3 = S.ds3h * w * fmaf(Pni, b.z, b.w);
-  const float tsum = -w * (a2 + a3);
+  const float tsum = pressure_term(S, d2, Pi, Pni, b);
   if (d2 > 0.0f) {
     const float s = tsum * rsqrtf(d2);
     f.x = fmaf(dx, s, f.x);
@@ -805,8 +935,6 @@ __device__ __forceinline__ void pressure_pair(const SceneDev& S, float3 p,
     f.y += tsum;  // dir = (0,1,0) for coincident particles (:414)
   }
 }
-
-
 
 // kLanes lanes per particle (tuning.particles_per_warp = 32 / kLanes): a
 // warp takes its tile's 32 particles in kLanes passes of 32 / kLanes; lane
@@ -893,6 +1021,100 @@ __global__ void k_pressure(const uint2* __restrict__ tiles, uint32_t ntiles,
   }
 }
 
+// Latency form for small launches (kCoopTiles): eight particles a warp,
+// four lanes a particle evaluate every fourth list entry each and leave (direction,
+// magnitude) in shared memory; one lane a component sums them in list order,
+// with the operations of pressure_pair, so the result is k_pressure's bit for bit
+// (16,384 particles 14 -> 10 us; with 8 instead of 32 particles a warp and the
+// terms staged it takes 2.3 times the plain form's instructions, which large
+// launches pay: 1M 93 -> 210 us).
+constexpr int kCoopTerms = kNbrCap + 1;  // float4 rows, shifted a bank group each
+constexpr int kCoopGather = 4;           // entries a lane has in flight
+
+// Component `comp` of the ordered sum of fma(direction, magnitude) over a row.
+__device__ __forceinline__ float coop_sum(const float4* row, uint32_t comp, uint32_t cnt) {
+  const float* p = reinterpret_cast<const float*>(row);
+  float f = 0.0f;
+#pragma unroll 4
+  for (uint32_t k = 0; k < cnt; ++k) f = fmaf(p[4u * k + comp], p[4u * k + 3u], f);
+  return f;
+}
+
+template <int kTables>
+__global__ void __launch_bounds__(kCoopBlock)
+k_pressure_coop(const uint2* __restrict__ tiles, uint32_t ntiles,
+                const SceneDev* __restrict__ scenes, const float4* __restrict__ pred,
+                const uint32_t* __restrict__ start, const uint32_t* __restrict__ cell_first,
+                const uint2* __restrict__ cell_tab, const float2* __restrict__ dens_a,
+                const float4* __restrict__ dens_b, const uint32_t* __restrict__ nbr,
+                const uint32_t* __restrict__ ncount, const float4* __restrict__ vel,
+                float4* __restrict__ rec_v, float4* __restrict__ dbg_accp) {
+  __shared__ float4 s_t[kCoopWarps][kCoopPer][kCoopTerms];
+  pdl_enter();
+  const uint32_t lane = lane_id();
+  const uint32_t pp = lane % kCoopPer, part = lane / kCoopPer;
+  float4* const row = s_t[threadIdx.x >> 5][pp];
+  for (uint32_t v = warp_id_global(); v < ntiles * kCoopSub; v += warps_total()) {
+    const uint2 tile = tiles[v / kCoopSub];
+    const uint32_t sub = v % kCoopSub * kCoopPer, len = tile_len(tile);
+    if (sub >= len) continue;
+    const SceneDev& S = scenes[tile_scene(tile)];
+    const bool live = sub + pp < len;
+    const uint32_t i = tile.y + min(sub + pp, len - 1u);
+    const float4 pi = pred[i];
+    const float3 p = make_float3(pi.x, pi.y, pi.z);
+    const float2 di = dens_a[i];
+    const float4 vi = vel[i];
+    const float Pi = (di.x - S.rho0) * S.k, Pni = di.y * S.kn;
+    const uint32_t cnt = live ? ncount[i] : 0u;
+    float3 f = make_float3(0.0f, 0.0f, 0.0f);
+    if (cnt <= kNbrCap) {
+      for (uint32_t k0 = part; k0 < cnt; k0 += 4u * kCoopGather) {
+        uint32_t j[kCoopGather];
+        float4 q[kCoopGather], b[kCoopGather];
+        load_nbr_batch<kCoopGather, 4>(nbr, i, k0, cnt, j);
+#pragma unroll
+        for (int u = 0; u < kCoopGather; ++u) {
+          if (k0 + 4u * u < cnt) {
+            q[u] = __ldg(pred + j[u]);
+            b[u] = __ldg(dens_b + j[u]);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < kCoopGather; ++u) {
+          if (k0 + 4u * u < cnt) {
+            const float dx = q[u].x - p.x, dy = q[u].y - p.y, dz = q[u].z - p.z;
+            const float d2 = dist2(dx, dy, dz);
+            const float tsum = pressure_term(S, d2, Pi, Pni, b[u]);
+            row[k0 + 4u * u] = d2 > 0.0f ? make_float4(dx, dy, dz, tsum * rsqrtf(d2))
+                                         : make_float4(0.0f, 1.0f, 0.0f, tsum);
+          }
+        }
+      }
+    } else if (part == 0) {
+      walk_runs<kTables>(S, start, cell_tab, cell_first[i], __float_as_uint(pi.w), pred,
+                         [&](uint32_t j, float4 q) {
+        if (j == i) return;
+        const float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
+        if (dist2(dx, dy, dz) <= S.cut_le)
+          pressure_pair(S, p, Pi, Pni, q, __ldg(dens_b + j), f);
+      });
+    }
+    __syncwarp();
+    const float fc = coop_sum(row, min(part, 2u), cnt <= kNbrCap ? cnt : 0u);
+    const float fx = __shfl_sync(kFull, fc, pp), fy = __shfl_sync(kFull, fc, kCoopPer + pp),
+                fz = __shfl_sync(kFull, fc, 2 * kCoopPer + pp);
+    if (cnt <= kNbrCap) f = make_float3(fx, fy, fz);
+    __syncwarp();  // the next slots rewrite the rows
+    if (!live || part != 0) continue;
+    const float inv_rho = 1.0f / di.x;
+    const float ax = f.x * inv_rho, ay = f.y * inv_rho, az = f.z * inv_rho;
+    store_rec(rec_v, i, pi,
+              make_float4(vi.x + ax * S.dt, vi.y + ay * S.dt, vi.z + az * S.dt, 0.f));
+    if (dbg_accp) dbg_accp[i] = make_float4(ax, ay, az, 0.0f);
+  }
+}
+
 // ------------------------------------------------ viscosity + integrate
 // CalculateViscosityForce (:424-464) over the neighbour list reading the
 // post-pressure snapshot (Jacobi); poly6 = (r^2 - d^2)^3 for dist < r. Then
@@ -911,6 +1133,39 @@ __device__ __forceinline__ void visc_pair(const SceneDev& S, float3 p,
     f.y = fmaf(vj.y - vi.y, w3, f.y);
     f.z = fmaf(vj.z - vi.z, w3, f.z);
   }
+}
+
+// The viscosity increment f of slot i, then the integration and the box
+// collision; with fuse_next also the key of the new state's prediction (S_next
+// is the same scene: its grid constants are read there, not kept in registers
+// through the sum).
+__device__ __forceinline__ void integrate(const SceneDev& S, const SceneDev& S_next, uint32_t i,
+                                          float4 vi, float3 f, float4* __restrict__ pos,
+                                          float4* __restrict__ vel, float4* __restrict__ out4,
+                                          int fuse_next, float4* __restrict__ dbg_velv,
+                                          uint32_t& key, uint32_t& cell, uint32_t& id, bool& bad) {
+  const float c = S.vscale * S.mu * S.dt;
+  float3 v = make_float3(vi.x + f.x * c, vi.y + f.y * c, vi.z + f.z * c);
+  if (dbg_velv) dbg_velv[i] = make_float4(v.x, v.y, v.z, 0.0f);
+  float4 x = pos[i];
+  x.x = __fadd_rn(x.x, __fmul_rn(v.x, S.dt));
+  x.y = __fadd_rn(x.y, __fmul_rn(v.y, S.dt));
+  x.z = __fadd_rn(x.z, __fmul_rn(v.z, S.dt));
+  // edgeDst = halfSize - |pos|; if <= 0 clamp to the wall and reflect.
+  if (S.hx - fabsf(x.x) <= 0.0f) { x.x = S.hx * copysign_or_zero(x.x); v.x *= S.ndamp; }
+  if (S.hy - fabsf(x.y) <= 0.0f) { x.y = S.hy * copysign_or_zero(x.y); v.y *= S.ndamp; }
+  if (S.hz - fabsf(x.z) <= 0.0f) { x.z = S.hz * copysign_or_zero(x.z); v.z *= S.ndamp; }
+  pos[i] = x;
+  const float4 v4 = make_float4(v.x, v.y, v.z, 0.0f);
+  vel[i] = v4;
+  bad = !(isfinite(x.x) && isfinite(x.y) && isfinite(x.z) &&
+          isfinite(v.x) && isfinite(v.y) && isfinite(v.z));
+  id = __float_as_uint(x.w);
+  if (out4) {
+    if (id < S.n) out4[S.base + id] = make_float4(x.x, x.y, x.z, 0.34f);
+    else bad = true;
+  }
+  if (fuse_next) predict_key(S_next, x, v4, key, cell);
 }
 
 // kLanes lanes per particle as in k_pressure.
@@ -976,29 +1231,8 @@ __global__ void k_visc_integrate(
         f.z += __shfl_xor_sync(kFull, f.z, 16);
       }
       if (live) {
-        const float c = S.vscale * S.mu * S.dt;
-        float3 v = make_float3(vi.x + f.x * c, vi.y + f.y * c, vi.z + f.z * c);
-        if (dbg_velv) dbg_velv[i] = make_float4(v.x, v.y, v.z, 0.0f);
-        float4 x = pos[i];
-        x.x = __fadd_rn(x.x, __fmul_rn(v.x, S.dt));
-        x.y = __fadd_rn(x.y, __fmul_rn(v.y, S.dt));
-        x.z = __fadd_rn(x.z, __fmul_rn(v.z, S.dt));
-        // edgeDst = halfSize - |pos|; if <= 0 clamp to the wall and reflect.
-        if (S.hx - fabsf(x.x) <= 0.0f) { x.x = S.hx * copysign_or_zero(x.x); v.x *= S.ndamp; }
-        if (S.hy - fabsf(x.y) <= 0.0f) { x.y = S.hy * copysign_or_zero(x.y); v.y *= S.ndamp; }
-        if (S.hz - fabsf(x.z) <= 0.0f) { x.z = S.hz * copysign_or_zero(x.z); v.z *= S.ndamp; }
-        pos[i] = x;
-        const float4 v4 = make_float4(v.x, v.y, v.z, 0.0f);
-        vel[i] = v4;
-        bad = !(isfinite(x.x) && isfinite(x.y) && isfinite(x.z) &&
-                isfinite(v.x) && isfinite(v.y) && isfinite(v.z));
-        id = __float_as_uint(x.w);
-        if (out4) {
-          if (id < S.n) out4[S.base + id] = make_float4(x.x, x.y, x.z, 0.34f);
-          else bad = true;
-        }
-        // the grid constants are read here, not kept in registers through the loop
-        if (fuse_next) predict_key(scenes[tile_scene(tile)], x, v4, key, cell);
+        integrate(S, scenes[tile_scene(tile)], i, vi, f, pos, vel, out4, fuse_next, dbg_velv, key,
+                  cell, id, bad);
       }
       if (fuse_next) {
         const uint32_t r = aggregated_rank(count, key, live);
@@ -1006,6 +1240,79 @@ __global__ void k_visc_integrate(
       }
       if (__any_sync(kFull, bad) && lane == 0) flag(status, kStatusNonFinite);
     }
+  }
+}
+
+// Latency form for small launches, as k_pressure_coop: the terms of visc_pair
+// by four lanes a particle, summed in list order.
+template <int kTables>
+__global__ void __launch_bounds__(kCoopBlock) k_visc_coop(
+    const uint2* __restrict__ tiles, uint32_t ntiles, const SceneDev* __restrict__ scenes,
+    const float4* __restrict__ pred, const uint32_t* __restrict__ start,
+    const uint32_t* __restrict__ cell_first, const uint2* __restrict__ cell_tab,
+    const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ ncount,
+    const float4* __restrict__ rec_v, float4* __restrict__ pos, float4* __restrict__ vel,
+    float4* __restrict__ out4, int fuse_next, uint32_t* __restrict__ count,
+    uint4* __restrict__ keyrank, float4* __restrict__ dbg_velv, uint32_t* status) {
+  __shared__ float4 s_t[kCoopWarps][kCoopPer][kCoopTerms];
+  pdl_enter();
+  const uint32_t lane = lane_id();
+  const uint32_t pp = lane % kCoopPer, part = lane / kCoopPer;
+  float4* const row = s_t[threadIdx.x >> 5][pp];
+  for (uint32_t v = warp_id_global(); v < ntiles * kCoopSub; v += warps_total()) {
+    const uint2 tile = tiles[v / kCoopSub];
+    const uint32_t sub = v % kCoopSub * kCoopPer, len = tile_len(tile);
+    if (sub >= len) continue;
+    const SceneDev& S = scenes[tile_scene(tile)];
+    const bool in_tile = sub + pp < len;
+    const uint32_t i = tile.y + min(sub + pp, len - 1u);
+    float4 pi, vi;
+    load_rec(rec_v, i, pi, vi);
+    const float3 p = make_float3(pi.x, pi.y, pi.z);
+    const uint32_t cnt = in_tile ? ncount[i] : 0u;
+    float3 f = make_float3(0.0f, 0.0f, 0.0f);
+    if (cnt <= kNbrCap) {
+      for (uint32_t k0 = part; k0 < cnt; k0 += 4u * kCoopGather) {
+        uint32_t j[kCoopGather];
+        float4 q[kCoopGather], vj[kCoopGather];
+        load_nbr_batch<kCoopGather, 4>(nbr, i, k0, cnt, j);
+#pragma unroll
+        for (int u = 0; u < kCoopGather; ++u)
+          if (k0 + 4u * u < cnt) load_rec(rec_v, j[u], q[u], vj[u]);
+#pragma unroll
+        for (int u = 0; u < kCoopGather; ++u) {
+          if (k0 + 4u * u < cnt) {
+            const float dx = q[u].x - p.x, dy = q[u].y - p.y, dz = q[u].z - p.z;
+            const float d2 = dist2(dx, dy, dz);
+            const float w = S.r2 - d2;
+            row[k0 + 4u * u] = d2 <= S.cut_lt
+                                   ? make_float4(vj[u].x - vi.x, vj[u].y - vi.y, vj[u].z - vi.z,
+                                                 w * w * w)
+                                   : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          }
+        }
+      }
+    } else if (part == 0) {
+      walk_runs<kTables>(S, start, cell_tab, cell_first[i], __float_as_uint(pi.w), pred,
+                         [&](uint32_t j, float4 q) {
+        if (j != i) visc_pair(S, p, vi, q, __ldg(rec_v + 2ull * j + 1), f);
+      });
+    }
+    __syncwarp();
+    const float fc = coop_sum(row, min(part, 2u), cnt <= kNbrCap ? cnt : 0u);
+    const float fx = __shfl_sync(kFull, fc, pp), fy = __shfl_sync(kFull, fc, kCoopPer + pp),
+                fz = __shfl_sync(kFull, fc, 2 * kCoopPer + pp);
+    if (cnt <= kNbrCap) f = make_float3(fx, fy, fz);
+    __syncwarp();  // the next slots rewrite the rows
+    const bool live = in_tile && part == 0u;
+    bool bad = false;
+    uint32_t key = 0, cell = 0, id = 0;
+    if (live) integrate(S, S, i, vi, f, pos, vel, out4, fuse_next, dbg_velv, key, cell, id, bad);
+    if (fuse_next) {
+      const uint32_t r = aggregated_rank(count, key, live);
+      if (live) keyrank[i] = make_uint4(key, r, cell, id);
+    }
+    if (__any_sync(kFull, bad) && lane == 0) flag(status, kStatusNonFinite);
   }
 }
 
@@ -1386,9 +1693,35 @@ cudaError_t launch_sort_reorder(const LaunchCtx& c, const Tiles& old_tiles,
   return e;
 }
 
+// Launches that take the latency forms (the walk and the lane-a-particle
+// force kernels wait on serial chains while most of the GPU idles). Measured
+// per substep, us, plain / latency form:
+//   density  16k 32 / 11, 37k 35 / 16, 65k 36 / 25 (a settled pool 21 / 19),
+//            90k 37 / 31 (pool 21 / 24), 131k 38 / 41
+//   pressure 16k 14 / 10, 28k 14 / 11, 33k 12 / 13, 45k 14 / 14, 65k 14 / 19
+//   viscosity alike
+// The results are the plain forms' bit for bit, so a scene steps alike in a
+// batch of any size. Tunings that choose another arithmetic (two lanes a
+// particle, the cell tile) keep their own kernels.
+constexpr uint32_t kRowsTiles = 2048;  // 65,536 particles
+constexpr uint32_t kCoopTiles = 900;   // 28,800 particles
+bool rows_form(const LaunchCtx& c, uint32_t ntiles) {
+  return c.cell_tile <= 1 && ntiles <= kRowsTiles;
+}
+bool coop_form(const LaunchCtx& c, uint32_t ntiles) {
+  return c.lanes == 1 && ntiles <= kCoopTiles;
+}
+
 cudaError_t launch_density(const LaunchCtx& c, const Tiles& tiles,
                            cudaStream_t st) {
   if (tiles.n == 0) return cudaSuccess;
+  if (rows_form(c, tiles.n))
+    return launch_pdl(c.pdl,
+                      c.tables == kTablesDirect    ? k_density_rows<kTablesDirect>
+                      : c.tables == kTablesBuckets ? k_density_rows<kTablesBuckets>
+                                                   : k_density_rows<kTablesMixed>,
+                      tiles.n, 32 * kRowWarps, st, tiles.d, tiles.n, c.scenes, c.pred, c.start,
+                      c.cell_first, c.cell_tab, c.dens_a, c.dens_b, c.nbr, c.ncount);
   const int b = c.block_nbr;
   const uint32_t g = grid_for(tiles.n, b, c.max_blocks);
   if (c.cell_tile <= 1)
@@ -1439,12 +1772,22 @@ auto visc_kernel(int gather, int lanes) {
 cudaError_t launch_pressure(const LaunchCtx& c, const Tiles& tiles,
                             cudaStream_t st) {
   if (tiles.n == 0) return cudaSuccess;
+  if (coop_form(c, tiles.n))
+    return launch_pdl(c.pdl,
+                      c.tables == kTablesDirect    ? k_pressure_coop<kTablesDirect>
+                      : c.tables == kTablesBuckets ? k_pressure_coop<kTablesBuckets>
+                                                   : k_pressure_coop<kTablesMixed>,
+                      grid_for(tiles.n * kCoopSub, kCoopBlock, c.max_blocks), kCoopBlock, st,
+                      tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab,
+                      c.dens_a, c.dens_b, c.nbr, c.ncount, c.vel2, c.rec_v, c.dbg_accp);
   const int b = c.block_force;
   auto kern = c.tables == kTablesDirect    ? pressure_kernel<kTablesDirect>(c.gather, c.lanes)
               : c.tables == kTablesBuckets ? pressure_kernel<kTablesBuckets>(c.gather, c.lanes)
                                            : pressure_kernel<kTablesMixed>(c.gather, c.lanes);
-  return launch_pdl(c.pdl, kern, grid_for(tiles.n, b, c.max_blocks), b, st, tiles.d,
-                    tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab,
+  // Started early beside k_density_rows' blocks this kernel would run with the
+  // L1 their shared memory leaves it (37k particles: 9 us a substep).
+  return launch_pdl(c.pdl && !rows_form(c, tiles.n), kern, grid_for(tiles.n, b, c.max_blocks), b,
+                    st, tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab,
                     c.dens_a, c.dens_b, c.nbr, c.ncount,
                     c.vel2, c.rec_v, c.dbg_accp);
 }
@@ -1453,6 +1796,15 @@ cudaError_t launch_visc_integrate(const LaunchCtx& c, const Tiles& tiles,
                                   int fuse_next, int write_out,
                                   cudaStream_t st) {
   if (tiles.n == 0) return cudaSuccess;
+  if (coop_form(c, tiles.n))
+    return launch_pdl(c.pdl,
+                      c.tables == kTablesDirect    ? k_visc_coop<kTablesDirect>
+                      : c.tables == kTablesBuckets ? k_visc_coop<kTablesBuckets>
+                                                   : k_visc_coop<kTablesMixed>,
+                      grid_for(tiles.n * kCoopSub, kCoopBlock, c.max_blocks), kCoopBlock, st,
+                      tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab, c.nbr,
+                      c.ncount, c.rec_v, c.pos2, c.vel2, write_out ? c.out4 : nullptr, fuse_next,
+                      c.count, c.keyrank, c.dbg_velv, c.status);
   const int b = c.block_force;
   auto kern = c.tables == kTablesDirect    ? visc_kernel<kTablesDirect>(c.gather, c.lanes)
               : c.tables == kTablesBuckets ? visc_kernel<kTablesBuckets>(c.gather, c.lanes)
