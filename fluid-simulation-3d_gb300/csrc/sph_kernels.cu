@@ -67,13 +67,23 @@ __device__ __forceinline__ void flag(uint32_t* status, uint32_t f) {
 
 // Programmatic dependent launch: the substep kernels are launched with
 // programmatic stream serialisation (launch_pdl), so each one is scheduled
-// while its predecessor's last wave runs. Every such kernel starts here: it
-// lets its own successor be scheduled, then waits for its predecessor to
-// complete with its memory visible (a hardware dependency, not a spin), so
-// nothing is read early. Without the launch attribute both are no-ops.
-__device__ __forceinline__ void pdl_enter() {
+// while its predecessor's last wave runs. Every such kernel first lets its
+// own successor be scheduled (pdl_launch), may then read what no kernel of a
+// step writes -- the tile table and the scene constants, uploaded before the
+// step began -- and waits for its predecessor to complete with its memory
+// visible (pdl_wait: a hardware dependency, not a spin) before it touches
+// anything else. Reading the tables before the wait takes two dependent loads
+// off the chain of each of the seven to eight kernels of a substep. Without the launch
+// attribute both are no-ops; a second wait returns at once.
+__device__ __forceinline__ void pdl_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_enter() {
+  pdl_launch();
+  pdl_wait();
 }
 
 // Entry k of slot i's neighbour list. Groups of 32 slots own kNbrCap rows of
@@ -229,11 +239,12 @@ __global__ void k_predict_hash(const uint2* __restrict__ tiles, uint32_t ntiles,
                                const float4* __restrict__ vel,
                                uint32_t* __restrict__ count,
                                uint4* __restrict__ keyrank) {
-  pdl_enter();
+  pdl_launch();
   const uint32_t lane = lane_id();
   for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const SceneDev S = scenes[tile_scene(tile)];  // registers, not reloads
+    pdl_wait();
     const uint32_t s = tile.y + lane;
     const bool live = lane < tile_len(tile);
     uint32_t key = 0, cell = 0, id = 0;
@@ -380,10 +391,11 @@ __global__ void k_scatter(const uint2* __restrict__ tiles, uint32_t ntiles,
                           const uint32_t* __restrict__ start, uint32_t total,
                           uint2* __restrict__ tmp_hi,
                           uint32_t* __restrict__ tmp_src, uint32_t* status) {
-  pdl_enter();
+  pdl_launch();
   const uint32_t lane = lane_id();
   for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
+    pdl_wait();
     const uint32_t s = tile.y + lane;
     if (lane >= tile_len(tile)) continue;
     const uint4 kr = keyrank[s];
@@ -412,11 +424,12 @@ __global__ void k_reorder(const uint2* __restrict__ tiles, uint32_t ntiles,
                           uint32_t* __restrict__ hash_s,
                           uint32_t* __restrict__ cell_first,
                           uint32_t src_limit, uint32_t* status) {
-  pdl_enter();
+  pdl_launch();
   const uint32_t lane = lane_id();
   for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const SceneDev S = scenes[tile_scene(tile)];  // registers, not reloads
+    pdl_wait();
     const uint32_t slot = tile.y + lane;
     if (lane >= tile_len(tile)) continue;
     const uint2 me = tmp_hi[slot];
@@ -481,9 +494,56 @@ __device__ __forceinline__ uint2 bucket_run(uint32_t cell, uint32_t b0,
 // keys; when their runs are adjacent in the layout (their buckets hold no
 // other cell -- the usual case inside the box) the row is stored as one run
 // flagged kRunMerged in its first entry (its other two entries are left
-// unwritten: a third of the table's stores, which the readers skip). Lanes take (cell, row)
-// pairs of the warp's tile in parallel; the warp's cell leaders are listed
-// in shared memory (kCellTableBlock threads per block).
+// unwritten: a third of the table's stores, which the readers skip).
+// cell_row: row w of the cell whose first slot is `slot`.
+__device__ __forceinline__ void cell_row(const SceneDev& S, uint32_t slot, uint32_t w, uint32_t kmax,
+                                         const uint32_t* __restrict__ hash_s,
+                                         const uint32_t* __restrict__ start,
+                                         uint2* __restrict__ cell_tab) {
+  const uint32_t dy = w / 3u - 1u, dz = w % 3u - 1u;  // mod 2^32
+  const uint32_t mid = __ldg(hash_s + slot) + dy * S.gwy + dz * S.gwz;
+  uint2* out = cell_tab + static_cast<uint64_t>(slot) * 27u + 3u * w;
+  // keys of mid - 1, mid, mid + 1: neighbours of mid's key modulo n,
+  // except across the 2^32 wrap of the index
+  const uint32_t km = fastmod(mid, S.fm, S.n);
+  const uint32_t kl = mid == 0u ? kmax : (km == 0u ? S.n - 1u : km - 1u);
+  const uint32_t kh = mid == 0xffffffffu ? 0u : (km + 1u == S.n ? 0u : km + 1u);
+  const uint32_t* st = start + S.tbase;
+  const uint32_t l0 = __ldg(st + kl), l1 = __ldg(st + kl + 1);
+  const uint32_t m0 = kl + 1u == km ? l1 : __ldg(st + km);
+  const uint32_t m1 = __ldg(st + km + 1);
+  const uint32_t h0 = kh == km + 1u ? m1 : __ldg(st + kh);
+  const uint32_t h1 = __ldg(st + kh + 1);
+  uint2 run[3];
+  run[0] = bucket_run(mid - 1u, l0, l1, hash_s);
+  run[1] = bucket_run(mid, m0, m1, hash_s);
+  run[2] = bucket_run(mid + 1u, h0, h1, hash_s);
+  uint32_t f = 0, e = 0;
+  bool any = false, adjacent = true;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (run[k].y == 0) continue;
+    if (!any) {
+      f = run[k].x;
+      e = f + run[k].y;
+      any = true;
+    } else if (run[k].x == e) {
+      e += run[k].y;
+    } else {
+      adjacent = false;
+    }
+  }
+  if (adjacent) {
+    out[0] = make_uint2(f, (e - f) | kRunMerged);
+  } else {
+    out[0] = run[0];
+    out[1] = run[1];
+    out[2] = run[2];
+  }
+}
+
+// Lanes take (cell, row) pairs of the warp's tile in parallel; the warp's
+// cell leaders are listed in shared memory (kCellTableBlock threads per block).
 constexpr int kCellTableBlock = 256;
 
 __global__ void __launch_bounds__(kCellTableBlock)
@@ -492,13 +552,14 @@ k_cell_table(const uint2* __restrict__ tiles, uint32_t ntiles,
              const uint32_t* __restrict__ hash_s,
              const uint32_t* __restrict__ cell_first,
              const uint32_t* __restrict__ start, uint2* __restrict__ cell_tab) {
-  pdl_enter();
+  pdl_launch();
   __shared__ uint8_t s_lead[kCellTableBlock / 32][32];
   uint8_t* lead = s_lead[threadIdx.x >> 5];
   const uint32_t lane = lane_id();
   for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const SceneDev S = scenes[tile_scene(tile)];  // registers, not reloads
+    pdl_wait();
     if (S.direct) continue;  // its rows come from the start table
     const uint32_t i = tile.y + lane;
     const bool live = lane < tile_len(tile);
@@ -510,49 +571,30 @@ k_cell_table(const uint2* __restrict__ tiles, uint32_t ntiles,
     const uint32_t kmax = fastmod(0xffffffffu, S.fm, S.n);  // key of 2^32 - 1
     for (uint32_t q = lane; q < pairs; q += 32) {
       const uint32_t c = q / 9u, w = q - c * 9u;
-      const uint32_t slot = tile.y + lead[c];
-      const uint32_t dy = w / 3u - 1u, dz = w % 3u - 1u;  // mod 2^32
-      const uint32_t mid = __ldg(hash_s + slot) + dy * S.gwy + dz * S.gwz;
-      uint2* out = cell_tab + static_cast<uint64_t>(slot) * 27u + 3u * w;
-      // keys of mid - 1, mid, mid + 1: neighbours of mid's key modulo n,
-      // except across the 2^32 wrap of the index
-      const uint32_t km = fastmod(mid, S.fm, S.n);
-      const uint32_t kl = mid == 0u ? kmax : (km == 0u ? S.n - 1u : km - 1u);
-      const uint32_t kh = mid == 0xffffffffu ? 0u : (km + 1u == S.n ? 0u : km + 1u);
-      const uint32_t* st = start + S.tbase;
-      const uint32_t l0 = __ldg(st + kl), l1 = __ldg(st + kl + 1);
-      const uint32_t m0 = kl + 1u == km ? l1 : __ldg(st + km);
-      const uint32_t m1 = __ldg(st + km + 1);
-      const uint32_t h0 = kh == km + 1u ? m1 : __ldg(st + kh);
-      const uint32_t h1 = __ldg(st + kh + 1);
-      uint2 run[3];
-      run[0] = bucket_run(mid - 1u, l0, l1, hash_s);
-      run[1] = bucket_run(mid, m0, m1, hash_s);
-      run[2] = bucket_run(mid + 1u, h0, h1, hash_s);
-      uint32_t f = 0, e = 0;
-      bool any = false, adjacent = true;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        if (run[k].y == 0) continue;
-        if (!any) {
-          f = run[k].x;
-          e = f + run[k].y;
-          any = true;
-        } else if (run[k].x == e) {
-          e += run[k].y;
-        } else {
-          adjacent = false;
-        }
-      }
-      if (adjacent) {
-        out[0] = make_uint2(f, (e - f) | kRunMerged);
-      } else {
-        out[0] = run[0];
-        out[1] = run[1];
-        out[2] = run[2];
-      }
+      cell_row(S, tile.y + lead[c], w, kmax, hash_s, start, cell_tab);
     }
     __syncwarp();  // the next tile rewrites the leader list
+  }
+}
+
+// Latency form for small launches: nine warps a tile, a row each, the lanes
+// that lead a cell at work (k_cell_table gives a warp up to nine such passes
+// one after another: 1,000 particles 11 us).
+__global__ void __launch_bounds__(288)
+k_cell_table_rows(const uint2* __restrict__ tiles, uint32_t ntiles,
+                  const SceneDev* __restrict__ scenes, const uint32_t* __restrict__ hash_s,
+                  const uint32_t* __restrict__ cell_first, const uint32_t* __restrict__ start,
+                  uint2* __restrict__ cell_tab) {
+  pdl_launch();
+  const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+  for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const uint2 tile = tiles[t];
+    const SceneDev S = scenes[tile_scene(tile)];
+    pdl_wait();
+    if (S.direct) continue;  // its rows come from the start table
+    const uint32_t i = tile.y + lane;
+    if (lane < tile_len(tile) && cell_first[i] == i)
+      cell_row(S, i, w, fastmod(0xffffffffu, S.fm, S.n), hash_s, start, cell_tab);
   }
 }
 
@@ -609,11 +651,12 @@ __global__ void __maxnreg__(32) k_density_walk(const uint2* __restrict__ tiles,
                                uint32_t* __restrict__ nbr,
                                uint32_t* __restrict__ ncount,
                                uint32_t nbr_step, uint32_t nbr_cap) {
-  pdl_enter();
+  pdl_launch();
   const uint32_t lane = lane_id();
   for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const SceneDev& S = scenes[tile_scene(tile)];
+    pdl_wait();
     if (lane >= tile_len(tile)) continue;
     const uint32_t i = tile.y + lane;
     const float4 me = pred[i];
@@ -668,7 +711,7 @@ constexpr int kRowWarps = 9;
 constexpr uint32_t kRowCap = 16;  // hits a queue holds
 
 template <int kTables>
-__global__ void __launch_bounds__(32 * kRowWarps)
+__global__ void __launch_bounds__(32 * kRowWarps, 4)  // the blocks an SM's shared memory holds
 k_density_rows(const uint2* __restrict__ tiles, uint32_t ntiles,
                const SceneDev* __restrict__ scenes, const float4* __restrict__ pred,
                const uint32_t* __restrict__ start, const uint32_t* __restrict__ cell_first,
@@ -678,20 +721,22 @@ k_density_rows(const uint2* __restrict__ tiles, uint32_t ntiles,
   __shared__ float2 s_hit[kRowWarps][kRowCap][32];
   __shared__ float s_w[kNbrCap][32];
   __shared__ uint32_t s_cnt[kRowWarps][32];
-  pdl_enter();
+  pdl_launch();
   const uint32_t lane = lane_id(), s = threadIdx.x >> 5;
   for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const uint2 tile = tiles[t];
     const SceneDev& S = scenes[tile_scene(tile)];
+    const float cut = S.cut_le, r = S.r;
+    const uint32_t row0 = S.tbase + (s / 3u - 1u) * S.gwy + (s % 3u - 1u) * S.gwz;
     const bool direct = kTables == kTablesDirect    ? true
                       : kTables == kTablesBuckets ? false
                                                   : S.direct != 0u;
+    pdl_wait();
     const bool live = lane < tile_len(tile);
     const uint32_t i = tile.y + (live ? lane : 0u);
     const float4 me = pred[i];
     const uint32_t cell = __float_as_uint(me.w);
     const uint32_t cf = kTables == kTablesDirect ? 0u : cell_first[i];
-    const float cut = S.cut_le, r = S.r;
     const float2 npxy = make_float2(-me.x, -me.y);
     uint32_t cnt = 0;
     auto run = [&](uint32_t j, uint32_t e) {
@@ -712,7 +757,7 @@ k_density_rows(const uint2* __restrict__ tiles, uint32_t ntiles,
     };
     if (live) {
       if (direct) {
-        const uint32_t k = S.tbase + cell + (s / 3u - 1u) * S.gwy + (s % 3u - 1u) * S.gwz;
+        const uint32_t k = row0 + cell;
         run(__ldg(start + k - 1), __ldg(start + k + 2));
       } else {
         const uint2* tab = cell_tab + static_cast<uint64_t>(cf) * 27u + s * 3u;
@@ -956,13 +1001,14 @@ __global__ void k_pressure(const uint2* __restrict__ tiles, uint32_t ntiles,
                            float4* __restrict__ rec_v,
                            float4* __restrict__ dbg_accp) {
   static_assert(kLanes == 1 || kLanes == 2, "one or two lanes per particle");
-  pdl_enter();
+  pdl_launch();
   const uint32_t lane = lane_id();
   constexpr uint32_t kPer = 32 / kLanes;  // particles per pass
   const uint32_t sub = lane / kPer;       // this lane's share of the list
   for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const SceneDev S = scenes[tile_scene(tile)];  // registers, not reloads
+    pdl_wait();
 #pragma unroll 1
     for (uint32_t h = 0; h < kLanes; ++h) {
       const uint32_t li = h * kPer + lane % kPer;
@@ -1050,7 +1096,7 @@ k_pressure_coop(const uint2* __restrict__ tiles, uint32_t ntiles,
                 const uint32_t* __restrict__ ncount, const float4* __restrict__ vel,
                 float4* __restrict__ rec_v, float4* __restrict__ dbg_accp) {
   __shared__ float4 s_t[kCoopWarps][kCoopPer][kCoopTerms];
-  pdl_enter();
+  pdl_launch();
   const uint32_t lane = lane_id();
   const uint32_t pp = lane % kCoopPer, part = lane / kCoopPer;
   float4* const row = s_t[threadIdx.x >> 5][pp];
@@ -1058,7 +1104,8 @@ k_pressure_coop(const uint2* __restrict__ tiles, uint32_t ntiles,
     const uint2 tile = tiles[v / kCoopSub];
     const uint32_t sub = v % kCoopSub * kCoopPer, len = tile_len(tile);
     if (sub >= len) continue;
-    const SceneDev& S = scenes[tile_scene(tile)];
+    const SceneDev S = scenes[tile_scene(tile)];
+    pdl_wait();
     const bool live = sub + pp < len;
     const uint32_t i = tile.y + min(sub + pp, len - 1u);
     const float4 pi = pred[i];
@@ -1181,13 +1228,14 @@ __global__ void k_visc_integrate(
     uint4* __restrict__ keyrank, float4* __restrict__ dbg_velv,
     uint32_t* status) {
   static_assert(kLanes == 1 || kLanes == 2, "one or two lanes per particle");
-  pdl_enter();
+  pdl_launch();
   const uint32_t lane = lane_id();
   constexpr uint32_t kPer = 32 / kLanes;  // particles per pass
   const uint32_t sub = lane / kPer;       // this lane's share of the list
   for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const SceneDev S = scenes[tile_scene(tile)];  // registers, not reloads
+    pdl_wait();
 #pragma unroll 1
     for (uint32_t h = 0; h < kLanes; ++h) {
       const uint32_t li = h * kPer + lane % kPer;
@@ -1255,7 +1303,7 @@ __global__ void __launch_bounds__(kCoopBlock) k_visc_coop(
     float4* __restrict__ out4, int fuse_next, uint32_t* __restrict__ count,
     uint4* __restrict__ keyrank, float4* __restrict__ dbg_velv, uint32_t* status) {
   __shared__ float4 s_t[kCoopWarps][kCoopPer][kCoopTerms];
-  pdl_enter();
+  pdl_launch();
   const uint32_t lane = lane_id();
   const uint32_t pp = lane % kCoopPer, part = lane / kCoopPer;
   float4* const row = s_t[threadIdx.x >> 5][pp];
@@ -1263,7 +1311,8 @@ __global__ void __launch_bounds__(kCoopBlock) k_visc_coop(
     const uint2 tile = tiles[v / kCoopSub];
     const uint32_t sub = v % kCoopSub * kCoopPer, len = tile_len(tile);
     if (sub >= len) continue;
-    const SceneDev& S = scenes[tile_scene(tile)];
+    const SceneDev S = scenes[tile_scene(tile)];
+    pdl_wait();
     const bool in_tile = sub + pp < len;
     const uint32_t i = tile.y + min(sub + pp, len - 1u);
     float4 pi, vi;
@@ -1672,27 +1721,6 @@ uint32_t scan_partials_needed(uint64_t len) {
   return static_cast<uint32_t>((len + kScanBlock - 1) / kScanBlock) + 1;
 }
 
-cudaError_t launch_sort_reorder(const LaunchCtx& c, const Tiles& old_tiles,
-                                const Tiles& new_tiles, uint32_t total,
-                                cudaStream_t st) {
-  cudaError_t e = cudaSuccess;
-  if (old_tiles.n)
-    e = launch_pdl(c.pdl, k_scatter, grid_for(old_tiles.n, c.block_misc, c.max_blocks),
-                   c.block_misc, st, old_tiles.d, old_tiles.n, c.keyrank, c.start,
-                   total, c.tmp_hi, c.tmp_src, c.status);
-  if (new_tiles.n && e == cudaSuccess) {
-    e = launch_pdl(c.pdl, k_reorder, grid_for(new_tiles.n, c.block_misc, c.max_blocks),
-                   c.block_misc, st, new_tiles.d, new_tiles.n, c.scenes, c.tmp_hi,
-                   c.tmp_src, c.start, c.pos, c.vel, c.pos2, c.vel2, c.pred,
-                   c.hash_s, c.cell_first, c.src_limit, c.status);
-    if (e == cudaSuccess && c.tables != kTablesDirect)
-      e = launch_pdl(c.pdl, k_cell_table, grid_for(new_tiles.n, kCellTableBlock, c.max_blocks),
-                     kCellTableBlock, st, new_tiles.d, new_tiles.n, c.scenes,
-                     c.hash_s, c.cell_first, c.start, c.cell_tab);
-  }
-  return e;
-}
-
 // Launches that take the latency forms (the walk and the lane-a-particle
 // force kernels wait on serial chains while most of the GPU idles). Measured
 // per substep, us, plain / latency form:
@@ -1710,6 +1738,31 @@ bool rows_form(const LaunchCtx& c, uint32_t ntiles) {
 }
 bool coop_form(const LaunchCtx& c, uint32_t ntiles) {
   return c.lanes == 1 && ntiles <= kCoopTiles;
+}
+
+cudaError_t launch_sort_reorder(const LaunchCtx& c, const Tiles& old_tiles,
+                                const Tiles& new_tiles, uint32_t total,
+                                cudaStream_t st) {
+  cudaError_t e = cudaSuccess;
+  if (old_tiles.n)
+    e = launch_pdl(c.pdl, k_scatter, grid_for(old_tiles.n, c.block_misc, c.max_blocks),
+                   c.block_misc, st, old_tiles.d, old_tiles.n, c.keyrank, c.start,
+                   total, c.tmp_hi, c.tmp_src, c.status);
+  if (new_tiles.n && e == cudaSuccess) {
+    e = launch_pdl(c.pdl, k_reorder, grid_for(new_tiles.n, c.block_misc, c.max_blocks),
+                   c.block_misc, st, new_tiles.d, new_tiles.n, c.scenes, c.tmp_hi,
+                   c.tmp_src, c.start, c.pos, c.vel, c.pos2, c.vel2, c.pred,
+                   c.hash_s, c.cell_first, c.src_limit, c.status);
+    if (e == cudaSuccess && c.tables != kTablesDirect)
+      e = new_tiles.n <= kRowsTiles
+              ? launch_pdl(c.pdl, k_cell_table_rows, new_tiles.n, 32 * kRowWarps, st, new_tiles.d,
+                           new_tiles.n, c.scenes, c.hash_s, c.cell_first, c.start, c.cell_tab)
+              : launch_pdl(c.pdl, k_cell_table,
+                           grid_for(new_tiles.n, kCellTableBlock, c.max_blocks), kCellTableBlock,
+                           st, new_tiles.d, new_tiles.n, c.scenes, c.hash_s, c.cell_first, c.start,
+                           c.cell_tab);
+  }
+  return e;
 }
 
 cudaError_t launch_density(const LaunchCtx& c, const Tiles& tiles,
