@@ -1228,14 +1228,13 @@ __global__ void k_visc_integrate(
     uint4* __restrict__ keyrank, float4* __restrict__ dbg_velv,
     uint32_t* status) {
   static_assert(kLanes == 1 || kLanes == 2, "one or two lanes per particle");
-  pdl_launch();
+  pdl_enter();  // (the early table read costs this kernel registers: 8.4M 599 -> 627 us)
   const uint32_t lane = lane_id();
   constexpr uint32_t kPer = 32 / kLanes;  // particles per pass
   const uint32_t sub = lane / kPer;       // this lane's share of the list
   for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const SceneDev S = scenes[tile_scene(tile)];  // registers, not reloads
-    pdl_wait();
 #pragma unroll 1
     for (uint32_t h = 0; h < kLanes; ++h) {
       const uint32_t li = h * kPer + lane % kPer;
