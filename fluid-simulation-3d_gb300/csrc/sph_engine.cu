@@ -27,6 +27,10 @@ template <class T> T* DeviceAlias(T* p) {
   return static_cast<T*>(a.devicePointer);
 }
 
+const float* Aligned16(const float* p) {
+  return (reinterpret_cast<std::uintptr_t>(p) & 15u) ? nullptr : p;
+}
+
 constexpr float kPiF = 3.14159265358979323846f;  // glm::pi<float>()
 
 template <class Pred> float LargestWith(float r, Pred ok) {
@@ -365,22 +369,24 @@ int Engine::Load(uint32_t id, const float* pos3, const float* vel3,
   carry_valid_ = false;  // a new state needs its own prediction
   const float* dp = pos3;
   const float* dv = vel3;
-  const float* hp = device_ptrs ? nullptr : DeviceAlias(pos3);
-  const float* hv = device_ptrs ? nullptr : DeviceAlias(vel3);
+  // Rows the import kernel can read itself: device arrays and, over the
+  // link, pinned host arrays, 16-byte aligned.
+  const float* rp = device_ptrs ? Aligned16(pos3) : DeviceAlias(pos3);
+  const float* rv = device_ptrs ? Aligned16(vel3) : DeviceAlias(vel3);
+  const bool rows = rp && (!vel3 || rv);
   // A single scene whose device constants and layout are current (a step
   // has run since the last change): the import also predicts the next
   // step's first substep with those constants, and that step uses it if its
   // dt and substeps are unchanged (the carry test in Step).
-  const bool predict = hp && (!vel3 || hv) && max_scenes_ == 1 && !scenes_dirty_ &&
+  const bool predict = rows && max_scenes_ == 1 && !scenes_dirty_ &&
                        uploaded_substeps_ > 0 && !layout_dirty_ &&
                        n_tiles_old_ == n_tiles_new_ && total_ == n;
-  if (hp && (!vel3 || hv)) {
-    // pinned host rows: the import kernel reads them over the link itself
+  if (rows) {
     if (predict && count_extent_)
       SPH_CUDA(cudaMemsetAsync(ctx_.count, 0, sizeof(uint32_t) * count_extent_, st),
                "histogram reset");
-    SPH_CUDA(launch_import_rows(old_base_[id], n, hp, hv, d_pos_[cur_], d_vel_[cur_],
-                                predict ? ctx_.scenes + id : nullptr, ctx_.count,
+    SPH_CUDA(launch_import_rows(old_base_[id], n, rp, rv, d_pos_[cur_], d_vel_[cur_],
+                                ctx_.dens_a, predict ? ctx_.scenes + id : nullptr, ctx_.count,
                                 ctx_.keyrank, st),
              "import kernel");
     if (predict) {
@@ -402,12 +408,9 @@ int Engine::Load(uint32_t id, const float* pos3, const float* vel3,
   } else if (!pos3) {
     dv = nullptr;
   }
-  if (!(hp && (!vel3 || hv)))
-    SPH_CUDA(launch_import(old_base_[id], n, dp, dv, d_pos_[cur_], d_vel_[cur_], st),
+  if (!rows)
+    SPH_CUDA(launch_import(old_base_[id], n, dp, dv, d_pos_[cur_], d_vel_[cur_], ctx_.dens_a, st),
              "import kernel");
-  // Densities are unknown until the next step.
-  SPH_CUDA(cudaMemsetAsync(ctx_.dens_a + old_base_[id], 0, sizeof(float2) * n, st),
-           "cudaMemsetAsync");
   debug_valid_ = false;
   return SPH_OK;
 }

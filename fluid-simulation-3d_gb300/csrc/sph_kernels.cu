@@ -1588,12 +1588,15 @@ __global__ void k_export_layout(uint32_t first, uint32_t n,
 }
 
 // Load caller-order AoS arrays into a scene's slots (identity layout).
+// The densities start at zero (unknown until the next step).
 __global__ void k_import(uint32_t first, uint32_t n,
                          const float* __restrict__ ipos,
                          const float* __restrict__ ivel,
-                         float4* __restrict__ pos, float4* __restrict__ vel) {
+                         float4* __restrict__ pos, float4* __restrict__ vel,
+                         float2* __restrict__ dens) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
+  dens[first + k] = make_float2(0.0f, 0.0f);
   pos[first + k] = ipos ? make_float4(ipos[3 * k], ipos[3 * k + 1],
                                       ipos[3 * k + 2], __uint_as_float(k))
                        : make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(k));
@@ -1602,10 +1605,10 @@ __global__ void k_import(uint32_t first, uint32_t n,
                         : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
-// Upload straight from host memory (pinned buffers the device can address,
-// read over the CPU link): the caller-order float3 rows of 32 consecutive
-// particles are 384 contiguous bytes, 24 float4. Each warp reads its chunk as
-// aligned float4 (the link's transactions stay full) and transposes it
+// Upload from rows the device addresses directly: its own memory, or pinned
+// host buffers read over the CPU link. The caller-order float3 rows of 32
+// consecutive particles are 384 contiguous bytes, 24 float4. Each warp reads its
+// chunk as aligned float4 (the link's transactions stay full) and transposes it
 // through shared memory; a partial last chunk goes by scalar loads, so
 // nothing outside the 3n floats is touched. The arrays must be 16-byte
 // aligned (checked by the launcher's caller).
@@ -1614,12 +1617,16 @@ constexpr int kXferWarps = kXferBlock / 32;
 
 // With `scene` the kernel also predicts the next step's first substep for
 // the imported state exactly as k_predict_hash would (key, arrival rank,
-// cell, caller index, and the histogram), so that step can skip it.
+// cell, caller index, and the histogram), so that step can skip it: device
+// uploads did that, the import and the zeroing of the densities in three
+// launches (1M: 8 + 3 + 20 us; a pass of one upload and step 800 -> 790 us,
+// 1,000 particles 50 -> 44, 8.4M 5.54 -> 5.46 ms).
 __global__ void __launch_bounds__(kXferBlock)
 k_import_rows(uint32_t first, uint32_t n, const float* __restrict__ ipos,
               const float* __restrict__ ivel, float4* __restrict__ pos,
-              float4* __restrict__ vel, const SceneDev* __restrict__ scene,
-              uint32_t* __restrict__ count, uint4* __restrict__ keyrank) {
+              float4* __restrict__ vel, float2* __restrict__ dens,
+              const SceneDev* __restrict__ scene, uint32_t* __restrict__ count,
+              uint4* __restrict__ keyrank) {
   __shared__ __align__(16) float s_rows[kXferWarps][2][96];
   const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
   const uint32_t k0 = (blockIdx.x * kXferWarps + w) * 32u;
@@ -1651,6 +1658,7 @@ k_import_rows(uint32_t first, uint32_t n, const float* __restrict__ ipos,
     if (ivel) v4 = make_float4(sv[3 * lane], sv[3 * lane + 1], sv[3 * lane + 2], 0.0f);
     pos[first + k] = p4;
     vel[first + k] = v4;
+    dens[first + k] = make_float2(0.0f, 0.0f);
   }
   if (scene) {  // every lane of the warp takes part (warp-aggregated atomics)
     const SceneDev S = *scene;
@@ -1929,21 +1937,21 @@ cudaError_t launch_ref_lookup(const LaunchCtx& c, const Tiles& new_tiles,
 }
 
 cudaError_t launch_import(uint32_t first, uint32_t n, const float* ipos,
-                          const float* ivel, float4* pos, float4* vel,
+                          const float* ivel, float4* pos, float4* vel, float2* dens,
                           cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  k_import<<<(n + 255) / 256, 256, 0, st>>>(first, n, ipos, ivel, pos, vel);
+  k_import<<<(n + 255) / 256, 256, 0, st>>>(first, n, ipos, ivel, pos, vel, dens);
   return cudaGetLastError();
 }
 
 cudaError_t launch_import_rows(uint32_t first, uint32_t n, const float* ipos,
-                               const float* ivel, float4* pos, float4* vel,
+                               const float* ivel, float4* pos, float4* vel, float2* dens,
                                const SceneDev* scene, uint32_t* count, uint4* keyrank,
                                cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   const uint32_t warps = (n + 31) / 32;
   k_import_rows<<<(warps + kXferWarps - 1) / kXferWarps, kXferBlock, 0, st>>>(
-      first, n, ipos, ivel, pos, vel, scene, count, keyrank);
+      first, n, ipos, ivel, pos, vel, dens, scene, count, keyrank);
   return cudaGetLastError();
 }
 

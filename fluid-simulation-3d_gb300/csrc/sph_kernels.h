@@ -145,15 +145,16 @@ cudaError_t launch_export_layout(uint32_t first, uint32_t n, const SceneDev* sce
 // buffers of `c`.
 cudaError_t launch_ref_lookup(const LaunchCtx& c, const Tiles& new_tiles,
                               uint32_t total, cudaStream_t st);
+// Both imports also zero the scene's densities.
 cudaError_t launch_import(uint32_t first, uint32_t n, const float* ipos,
-                          const float* ivel, float4* pos, float4* vel,
+                          const float* ivel, float4* pos, float4* vel, float2* dens,
                           cudaStream_t st);
-// The same import reading host memory the device addresses directly (pinned
-// buffers, 16-byte aligned): rows move as aligned float4 per warp. With
-// `scene` (the scene's device constants) it also writes the next step's
+// The same import for 16-byte aligned rows the device addresses directly (its
+// own memory or pinned host buffers): rows move as aligned float4 per warp.
+// With `scene` (the scene's device constants) it also writes the next step's
 // first prediction (keyrank, histogram in count) as k_predict_hash does.
 cudaError_t launch_import_rows(uint32_t first, uint32_t n, const float* ipos,
-                               const float* ivel, float4* pos, float4* vel,
+                               const float* ivel, float4* pos, float4* vel, float2* dens,
                                const SceneDev* scene, uint32_t* count, uint4* keyrank,
                                cudaStream_t st);
 
