@@ -743,23 +743,30 @@ int Engine::Render(uint32_t id, const sph_view& v, uint8_t* rgba, float* depth,
     return Fail(SPH_ERR_INVALID, "scale must be positive and finite");
   for (float x : v.view_proj)
     if (!std::isfinite(x)) return Fail(SPH_ERR_INVALID, "view_proj must be finite");
-  if (pixels > render_pixels_) {
-    cudaFree(d_rkeys_);
-    cudaFree(d_rrgba_);
-    cudaFree(d_rdepth_);
-    d_rkeys_ = nullptr;
-    d_rrgba_ = nullptr;
-    d_rdepth_ = nullptr;
-    render_pixels_ = 0;
-    cudaError_t e = Alloc(&d_rkeys_, pixels);
-    if (e == cudaSuccess) e = Alloc(&d_rrgba_, pixels);
-    if (e == cudaSuccess) e = Alloc(&d_rdepth_, pixels);
-    if (e != cudaSuccess) {
+  // Pinned, 16-byte aligned outputs are resolved straight into; other host
+  // memory gets copies of images resolved on the device.
+  uint32_t* hc = reinterpret_cast<uint32_t*>(DeviceAlias(rgba));
+  float* hz = DeviceAlias(depth);
+  const bool direct = (rgba || depth) && (!rgba || hc) && (!depth || hz);
+  auto grow = [&](auto** p, uint64_t* have) {
+    if (pixels <= *have) return true;
+    cudaFree(*p);
+    *p = nullptr;
+    *have = 0;
+    if (Alloc(p, pixels) != cudaSuccess) {
       cudaGetLastError();
-      return Fail(SPH_ERR_NOMEM, "render buffers do not fit the device");
+      return false;
     }
-    render_pixels_ = pixels;
+    *have = pixels;
+    return true;
+  };
+  const uint64_t keys_before = render_pixels_;
+  if (!grow(&d_rkeys_, &render_pixels_) ||
+      (!direct && (!grow(&d_rrgba_, &rgba_pixels_) || !grow(&d_rdepth_, &depth_pixels_)))) {
+    render_empty_ = render_empty_ && render_pixels_ == keys_before;
+    return Fail(SPH_ERR_NOMEM, "render buffers do not fit the device");
   }
+  if (render_pixels_ != keys_before) render_empty_ = false;
   if (!d_rcolour_) SPH_CUDA(Alloc(&d_rcolour_, capacity_), "cudaMalloc");
   RenderView rv{};
   for (int k = 0; k < 16; ++k) rv.vp[k] = v.view_proj[k];
@@ -776,13 +783,18 @@ int Engine::Render(uint32_t id, const sph_view& v, uint8_t* rgba, float* depth,
     const float c = std::fmin(std::fmax(v.clear[k], 0.0f), 1.0f) * 255.0f;
     rv.clear |= static_cast<uint32_t>(std::lrint(c)) << (8 * k);
   }
+  if (!render_empty_)
+    SPH_CUDA(cudaMemsetAsync(d_rkeys_, 0xff, sizeof(unsigned long long) * render_pixels_, st),
+             "clear image keys");
+  render_empty_ = false;  // until this frame's resolve is queued
   SPH_CUDA(launch_render(old_base_[id], scenes_[id].n, d_pos_[cur_], d_vel_[cur_], rv,
-                         d_rkeys_, d_rcolour_, d_rrgba_, d_rdepth_, st),
+                         d_rkeys_, d_rcolour_, direct ? hc : d_rrgba_, direct ? hz : d_rdepth_, st),
            "render kernels");
-  if (rgba)
+  render_empty_ = true;
+  if (rgba && !direct)
     SPH_CUDA(cudaMemcpyAsync(rgba, d_rrgba_, 4 * pixels, cudaMemcpyDeviceToHost, st),
              "download image");
-  if (depth)
+  if (depth && !direct)
     SPH_CUDA(cudaMemcpyAsync(depth, d_rdepth_, 4 * pixels, cudaMemcpyDeviceToHost, st),
              "download depth");
   SPH_CUDA(cudaStreamSynchronize(st), "cudaStreamSynchronize");

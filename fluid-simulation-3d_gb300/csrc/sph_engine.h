@@ -158,12 +158,15 @@ class Engine {
   void* d_dbg_scratch_ = nullptr;
 
   // render buffers, grown on demand: (depth, index) keys, RGBA8 and depth per
-  // pixel, colour per particle
+  // pixel (the images only for outputs the resolve cannot write itself),
+  // colour per particle
   unsigned long long* d_rkeys_ = nullptr;
   uint32_t* d_rrgba_ = nullptr;
   float* d_rdepth_ = nullptr;
   uint32_t* d_rcolour_ = nullptr;
-  uint64_t render_pixels_ = 0;
+  uint64_t render_pixels_ = 0, rgba_pixels_ = 0, depth_pixels_ = 0;
+  bool render_empty_ = false;  // every key of the buffer is empty (a resolved
+                               // frame leaves it so)
 
   sph_tuning tuning_{128, 1, 32, 2, 0, 0};
   int sm_count_ = 0;

@@ -187,20 +187,40 @@ __global__ void k_splat(uint32_t first, uint32_t n, const float4* __restrict__ p
   }
 }
 
-// Thread per pixel: the winning particle's colour and depth, else the clear
-// colour and depth 1.
-__global__ void k_resolve(uint32_t pixels, const unsigned long long* __restrict__ keys,
+// Thread per four pixels: the winning particle's colour and depth, else the
+// clear colour and depth 1, as 16-byte words; a covered key is put back to
+// empty for the next frame (no clear of the whole buffer). The outputs may be
+// pinned host memory: the words then go over the link from here, which bounds
+// the frame (1080p, 16.6 MB, 131,072 particles: 117 us; 136 us when the keys
+// were cleared, the image resolved on the device and copied).
+__global__ void k_resolve(uint32_t pixels, unsigned long long* __restrict__ keys,
                           const uint32_t* __restrict__ colours, uint32_t clear,
                           uint32_t* __restrict__ rgba, float* __restrict__ depth) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
   if (i >= pixels) return;
-  const unsigned long long key = keys[i];
-  if (key == ~0ull) {
-    rgba[i] = clear;
-    depth[i] = 1.0f;
+  const uint32_t m = min(4u, pixels - i);
+  uint32_t c[4];
+  float z[4];
+#pragma unroll
+  for (uint32_t u = 0; u < 4; ++u) {
+    c[u] = clear;
+    z[u] = 1.0f;
+    if (u >= m) continue;
+    const unsigned long long key = keys[i + u];
+    if (key != ~0ull) {
+      c[u] = colours[static_cast<uint32_t>(key)];
+      z[u] = __uint_as_float(static_cast<uint32_t>(key >> 32));
+      keys[i + u] = ~0ull;
+    }
+  }
+  if (m == 4u) {
+    if (rgba) *reinterpret_cast<uint4*>(rgba + i) = make_uint4(c[0], c[1], c[2], c[3]);
+    if (depth) *reinterpret_cast<float4*>(depth + i) = make_float4(z[0], z[1], z[2], z[3]);
   } else {
-    rgba[i] = colours[static_cast<uint32_t>(key)];
-    depth[i] = __uint_as_float(static_cast<uint32_t>(key >> 32));
+    for (uint32_t u = 0; u < m; ++u) {
+      if (rgba) rgba[i + u] = c[u];
+      if (depth) depth[i + u] = z[u];
+    }
   }
 }
 
@@ -210,15 +230,13 @@ cudaError_t launch_render(uint32_t first, uint32_t n, const float4* pos, const f
                           const RenderView& view, unsigned long long* keys,
                           uint32_t* colours, uint32_t* rgba, float* depth,
                           cudaStream_t st) {
-  const uint64_t pixels = static_cast<uint64_t>(view.width) * view.height;
-  cudaError_t e = cudaMemsetAsync(keys, 0xff, sizeof(unsigned long long) * pixels, st);
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
   if (n) {
     k_splat<<<(n + 255) / 256, 256, 0, st>>>(first, n, pos, vel, view, keys, colours);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
-  const uint32_t px = static_cast<uint32_t>(pixels);
-  k_resolve<<<(px + 255) / 256, 256, 0, st>>>(px, keys, colours, view.clear, rgba, depth);
+  const uint32_t px = view.width * view.height;
+  k_resolve<<<(px + 1023) / 1024, 256, 0, st>>>(px, keys, colours, view.clear, rgba, depth);
   return cudaGetLastError();
 }
 

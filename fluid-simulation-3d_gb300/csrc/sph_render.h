@@ -19,9 +19,11 @@ struct RenderView {
   uint32_t clear;          // clear colour, RGBA8
 };
 
-// Clears keys[W*H], splats the scene's slots [first, first + n) of
-// (pos, vel) -- pos.w holds the caller index -- and resolves rgba[W*H] and
-// depth[W*H]; colours[n] receives every particle's colour by caller index.
+// Splats the scene's slots [first, first + n) of (pos, vel) -- pos.w holds the
+// caller index -- into keys[W*H], which must be empty (all ones) and is left so,
+// and resolves rgba[W*H] and depth[W*H] (16-byte aligned device or device-
+// mapped host memory, either may be nullptr); colours[n] receives every
+// particle's colour by caller index.
 cudaError_t launch_render(uint32_t first, uint32_t n, const float4* pos, const float4* vel,
                           const RenderView& view, unsigned long long* keys,
                           uint32_t* colours, uint32_t* rgba, float* depth,
