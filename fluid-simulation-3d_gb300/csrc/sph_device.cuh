@@ -6,8 +6,9 @@
 //   pred[P]             float4 (predicted position, cell index as raw bits)
 //   dens_a[P]           float2 (density, near density)
 //   dens_b[P]           float4 (1/rho, P/rho, 1/rho_n, Pn/rho_n)
-//   rec_v[2P]           32-byte records (pred, post-pressure velocity): the
-//                       Jacobi snapshot the viscosity pass reads
+//   rec_v[2P]           (pred, post-pressure velocity): the Jacobi snapshot the
+//                       viscosity pass reads; P float4 (x, y, z, vx) and P
+//                       float2 (vy, vz), or 32-byte records (latency forms)
 //   keyrank[P]          uint4 (global key, arrival rank in the key bucket,
 //                       cell index, particle index)
 //   tmp_hi[P], tmp_src[P] bucketed (cell index, particle index) and source

@@ -234,6 +234,7 @@ int Engine::Init() {
   SPH_CUDA(cudaMemset(d_out4_, 0, C * sizeof(float4)), "cudaMemset");
   ctx_.scenes = d_scenes_;
   ctx_.out4 = d_out4_;
+  ctx_.rec_b = reinterpret_cast<float2*>(ctx_.rec_v + C);
   ctx_.status = d_status_;
   return SPH_OK;
 }
@@ -525,6 +526,7 @@ int Engine::RunSubsteps(int substeps, cudaStream_t st, bool carry) {
     c.vel2 = d_vel_[1 - cur];
     const bool dbg = debug_ && ss == 0;
     c.dbg_accp = dbg ? d_dbg_accp_ : nullptr;
+    c.dbg_velp = dbg ? d_dbg_velp_ : nullptr;
     c.dbg_velv = dbg ? d_dbg_velv_ : nullptr;
     const Tiles& first = ss == 0 ? told : tnew;
     cudaEvent_t* ev = profile_ ? &prof_ev_[ss * kPhaseEvents] : nullptr;
@@ -552,10 +554,6 @@ int Engine::RunSubsteps(int substeps, cudaStream_t st, bool carry) {
     if (e == cudaSuccess)
       e = launch_visc_integrate(c, tnew, 1, ss + 1 == substeps ? 1 : 0, st);
     mark(5);
-    if (e == cudaSuccess && dbg)
-      e = cudaMemcpy2DAsync(d_dbg_velp_, sizeof(float4), c.rec_v + 1,
-                            2 * sizeof(float4), sizeof(float4), total_,
-                            cudaMemcpyDeviceToDevice, st);
     if (e != cudaSuccess) return CudaFail(e, "substep launch");
     cur = 1 - cur;
   }

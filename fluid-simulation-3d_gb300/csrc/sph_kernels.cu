@@ -98,8 +98,26 @@ __device__ __forceinline__ uint64_t nbr_index(uint32_t i, uint32_t k) {
   return static_cast<uint64_t>(i & ~31u) * kNbrCap + k * 32u + (i & 31u);
 }
 
-// 32-byte particle records (rec_v): two float4 halves that a neighbour
-// gather fetches with one 256-bit load from one sector.
+// The viscosity pass's particle records, (predicted position, post-pressure
+// velocity), six floats. The plain force kernels keep them as a float4 (x, y,
+// z, vx) and a float2 (vy, vz): their gathers are bound by the L1 data pipe,
+// which 24 B a neighbour load less than one padded 32-byte record (one
+// 256-bit load): viscosity at 1M 91 -> 83 us, at 8.4M 599 -> 585 us. The
+// latency forms, which wait on loads and not on the pipe, take the 32-byte
+// record and half the loads (16,384 particles: 2 us a substep).
+__device__ __forceinline__ void load_state(const float4* __restrict__ rec,
+                                           const float2* __restrict__ rec_b, uint32_t j,
+                                           float4& a, float4& b) {
+  const float4 x = __ldg(rec + j);
+  const float2 y = __ldg(rec_b + j);
+  a = make_float4(x.x, x.y, x.z, 0.0f);
+  b = make_float4(x.w, y.x, y.y, 0.0f);
+}
+__device__ __forceinline__ void store_state(float4* __restrict__ rec, float2* __restrict__ rec_b,
+                                            uint32_t i, float4 a, float4 b) {
+  rec[i] = make_float4(a.x, a.y, a.z, b.x);
+  rec_b[i] = make_float2(b.y, b.z);
+}
 __device__ __forceinline__ void load_rec(const float4* __restrict__ rec,
                                          uint32_t j, float4& a, float4& b) {
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -1012,8 +1030,9 @@ __global__ void k_pressure(const uint2* __restrict__ tiles, uint32_t ntiles,
                            const uint32_t* __restrict__ nbr,
                            const uint32_t* __restrict__ ncount,
                            const float4* __restrict__ vel,
-                           float4* __restrict__ rec_v,
-                           float4* __restrict__ dbg_accp) {
+                           float4* __restrict__ rec_v, float2* __restrict__ rec_b,
+                           float4* __restrict__ dbg_accp,
+                           float4* __restrict__ dbg_velp) {
   static_assert(kLanes == 1 || kLanes == 2, "one or two lanes per particle");
   pdl_launch();
   const uint32_t lane = lane_id();
@@ -1073,10 +1092,12 @@ __global__ void k_pressure(const uint2* __restrict__ tiles, uint32_t ntiles,
       const float inv_rho = 1.0f / di.x;
       const float ax = f.x * inv_rho, ay = f.y * inv_rho, az = f.z * inv_rho;
       const float4 v = vel[i];
-      // viscosity record rec_v[i] = (predicted position, post-pressure velocity)
-      store_rec(rec_v, i, pi,
-                make_float4(v.x + ax * S.dt, v.y + ay * S.dt, v.z + az * S.dt, 0.f));
-      if (dbg_accp) dbg_accp[i] = make_float4(ax, ay, az, 0.0f);
+      const float4 vp = make_float4(v.x + ax * S.dt, v.y + ay * S.dt, v.z + az * S.dt, 0.f);
+      store_state(rec_v, rec_b, i, pi, vp);
+      if (dbg_accp) {
+        dbg_accp[i] = make_float4(ax, ay, az, 0.0f);
+        dbg_velp[i] = vp;
+      }
     }
   }
 }
@@ -1108,7 +1129,8 @@ k_pressure_coop(const uint2* __restrict__ tiles, uint32_t ntiles,
                 const uint2* __restrict__ cell_tab, const float2* __restrict__ dens_a,
                 const float4* __restrict__ dens_b, const uint32_t* __restrict__ nbr,
                 const uint32_t* __restrict__ ncount, const float4* __restrict__ vel,
-                float4* __restrict__ rec_v, float4* __restrict__ dbg_accp) {
+                float4* __restrict__ rec_v, float4* __restrict__ dbg_accp,
+                float4* __restrict__ dbg_velp) {
   __shared__ float4 s_t[kCoopWarps][kCoopPer][kCoopTerms];
   pdl_launch();
   const uint32_t lane = lane_id();
@@ -1170,9 +1192,12 @@ k_pressure_coop(const uint2* __restrict__ tiles, uint32_t ntiles,
     if (!live || part != 0) continue;
     const float inv_rho = 1.0f / di.x;
     const float ax = f.x * inv_rho, ay = f.y * inv_rho, az = f.z * inv_rho;
-    store_rec(rec_v, i, pi,
-              make_float4(vi.x + ax * S.dt, vi.y + ay * S.dt, vi.z + az * S.dt, 0.f));
-    if (dbg_accp) dbg_accp[i] = make_float4(ax, ay, az, 0.0f);
+    const float4 vp = make_float4(vi.x + ax * S.dt, vi.y + ay * S.dt, vi.z + az * S.dt, 0.f);
+    store_rec(rec_v, i, pi, vp);
+    if (dbg_accp) {
+      dbg_accp[i] = make_float4(ax, ay, az, 0.0f);
+      dbg_velp[i] = vp;
+    }
   }
 }
 
@@ -1237,6 +1262,7 @@ __global__ void k_visc_integrate(
     const uint32_t* __restrict__ start,
     const uint32_t* __restrict__ cell_first, const uint2* __restrict__ cell_tab,
     const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ ncount, const float4* __restrict__ rec_v,
+    const float2* __restrict__ rec_b,
     float4* __restrict__ pos, float4* __restrict__ vel,
     float4* __restrict__ out4, int fuse_next, uint32_t* __restrict__ count,
     uint4* __restrict__ keyrank, float4* __restrict__ dbg_velv,
@@ -1260,7 +1286,7 @@ __global__ void k_visc_integrate(
       float4 pi, vi;
       float3 f = make_float3(0.0f, 0.0f, 0.0f);
       if (in_tile) {
-        load_rec(rec_v, i, pi, vi);
+        load_state(rec_v, rec_b, i, pi, vi);
         const float3 p = make_float3(pi.x, pi.y, pi.z);
         const uint32_t cnt = ncount[i];
         if (cnt <= kNbrCap) {
@@ -1274,15 +1300,18 @@ __global__ void k_visc_integrate(
             if (k0 + kLanes * kGather < cnt)
               load_nbr_batch<kGather, kLanes>(nbr, i, k0 + kLanes * kGather, cnt, jn);
 #pragma unroll
-            for (int u = 0; u < kGather; ++u) load_rec(rec_v, j[u], q[u], vj[u]);
+            for (int u = 0; u < kGather; ++u) load_state(rec_v, rec_b, j[u], q[u], vj[u]);
 #pragma unroll
             for (int u = 0; u < kGather; ++u)
               if (k0 + kLanes * u < cnt) visc_pair(S, p, vi, q[u], vj[u], f);
           }
         } else if (sub == 0) {
-          walk_runs<kTables>(S, start, cell_tab, cell_first[i], __float_as_uint(pi.w), pred,
+          walk_runs<kTables>(S, start, cell_tab, cell_first[i], __float_as_uint(pred[i].w), pred,
                              [&](uint32_t j, float4 q) {
-            if (j != i) visc_pair(S, p, vi, q, __ldg(rec_v + 2ull * j + 1), f);
+            if (j == i) return;
+            float4 a, b;
+            load_state(rec_v, rec_b, j, a, b);
+            visc_pair(S, p, vi, q, b, f);
           });
         }
       }
@@ -1856,7 +1885,8 @@ cudaError_t launch_pressure(const LaunchCtx& c, const Tiles& tiles,
                                                    : k_pressure_coop<kTablesMixed>,
                       grid_for(tiles.n * kCoopSub, kCoopBlock, c.max_blocks), kCoopBlock, st,
                       tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab,
-                      c.dens_a, c.dens_b, c.nbr, c.ncount, c.vel2, c.rec_v, c.dbg_accp);
+                      c.dens_a, c.dens_b, c.nbr, c.ncount, c.vel2, c.rec_v, c.dbg_accp,
+                      c.dbg_velp);
   const int b = c.block_force;
   auto kern = c.tables == kTablesDirect    ? pressure_kernel<kTablesDirect>(c.gather, c.lanes)
               : c.tables == kTablesBuckets ? pressure_kernel<kTablesBuckets>(c.gather, c.lanes)
@@ -1866,7 +1896,7 @@ cudaError_t launch_pressure(const LaunchCtx& c, const Tiles& tiles,
   return launch_pdl(c.pdl && !rows_form(c, tiles.n), kern, grid_for(tiles.n, b, c.max_blocks), b,
                     st, tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab,
                     c.dens_a, c.dens_b, c.nbr, c.ncount,
-                    c.vel2, c.rec_v, c.dbg_accp);
+                    c.vel2, c.rec_v, c.rec_b, c.dbg_accp, c.dbg_velp);
 }
 
 cudaError_t launch_visc_integrate(const LaunchCtx& c, const Tiles& tiles,
@@ -1888,7 +1918,7 @@ cudaError_t launch_visc_integrate(const LaunchCtx& c, const Tiles& tiles,
                                            : visc_kernel<kTablesMixed>(c.gather, c.lanes);
   return launch_pdl(c.pdl, kern, grid_for(tiles.n, b, c.max_blocks), b, st, tiles.d,
                     tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab, c.nbr,
-                    c.ncount, c.rec_v, c.pos2, c.vel2,
+                    c.ncount, c.rec_v, c.rec_b, c.pos2, c.vel2,
                     write_out ? c.out4 : nullptr, fuse_next, c.count, c.keyrank,
                     c.dbg_velv, c.status);
 }

@@ -48,7 +48,10 @@ struct LaunchCtx {
   float4* pos2 = nullptr;  // state B (written by the reorder)
   float4* vel2 = nullptr;
   float4* pred = nullptr;
-  float4* rec_v = nullptr;  // 2 per slot: (pred, post-pressure velocity)
+  float4* rec_v = nullptr;  // 2 per slot: (pred, post-pressure velocity), as
+                            // 32-byte records (latency forms) or as the first
+                            // of the two float4 per slot and rec_b
+  float2* rec_b = nullptr;  // in rec_v, behind its first float4 of every slot
   float2* dens_a = nullptr;
   float4* dens_b = nullptr;  // (1/rho, P/rho, 1/rho_n, Pn/rho_n) per slot
   uint4* keyrank = nullptr;   // (key, arrival rank, cell, id) per old slot
@@ -71,6 +74,7 @@ struct LaunchCtx {
   float4* out4 = nullptr;
   uint32_t* status = nullptr;
   float4* dbg_accp = nullptr;   // captured substep: per-slot intermediates
+  float4* dbg_velp = nullptr;
   float4* dbg_velv = nullptr;
   // captured substep: the reference's spatial lookup (launch_ref_lookup)
   uint32_t* dbg_hash = nullptr;     // HashCell per particle (base + index)
