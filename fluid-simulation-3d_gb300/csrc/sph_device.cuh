@@ -3,7 +3,8 @@
 // Layout in HBM (one engine, S scenes concatenated, capacity P particles):
 //   pos[P], vel[P]      float4 state in the current sorted layout; pos.w holds
 //                       the particle's index in its scene as raw bits
-//   pred[P]             float4 (predicted position, cell index as raw bits)
+//   pred[P]             float4 (predicted position, cell index as raw bits),
+//                       and kPredPad slots more
 //   dens_a[P]           float2 (density, near density)
 //   dens_b[P]           float4 (1/rho, P/rho, 1/rho_n, Pn/rho_n)
 //   rec_v[2P]           (pred, post-pressure velocity): the Jacobi snapshot the
@@ -48,6 +49,10 @@ constexpr uint32_t kHashZ = 440817757u;
 
 // Particles per tile: one warp. Tiles never straddle scenes.
 constexpr int kTile = 32;
+
+// Slots past the last whose predicted position a batch of candidate loads may
+// read (and drop).
+constexpr uint32_t kPredPad = 3;
 
 // Neighbour-list entries per particle (pairs with dist <= r); a particle with
 // more neighbours is handled by the walk of its cells in the force passes.

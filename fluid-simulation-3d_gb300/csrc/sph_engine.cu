@@ -204,7 +204,7 @@ int Engine::Init() {
     chk(Alloc(&d_pos_[b], C));
     chk(Alloc(&d_vel_[b], C));
   }
-  chk(Alloc(&ctx_.pred, C));
+  chk(Alloc(&ctx_.pred, C + kPredPad));
   chk(Alloc(&ctx_.rec_v, 2 * C));
   chk(Alloc(&ctx_.dens_a, C));
   chk(Alloc(&ctx_.dens_b, C));
@@ -229,6 +229,7 @@ int Engine::Init() {
                : CudaFail(e, "cudaMalloc");
   }
   SPH_CUDA(cudaMemset(ctx_.count, 0, T * sizeof(uint32_t)), "cudaMemset");
+  SPH_CUDA(cudaMemset(ctx_.pred + C, 0, kPredPad * sizeof(float4)), "cudaMemset");
   SPH_CUDA(cudaMemset(ctx_.dens_a, 0, C * sizeof(float2)), "cudaMemset");
   SPH_CUDA(cudaMemset(d_status_, 0, sizeof(uint32_t)), "cudaMemset");
   SPH_CUDA(cudaMemset(d_out4_, 0, C * sizeof(float4)), "cudaMemset");

@@ -663,63 +663,107 @@ __device__ __forceinline__ void density_store(const SceneDev& S, uint32_t i,
 // Thread-per-particle form in one pass: each lane walks its cell's runs,
 // classifies every candidate on the reference's exact d2 and accumulates the
 // density and its list as it goes. Lanes of one cell walk identical runs, so
-// their loads coincide. The walk is issue-bound: the cutoff and radius sit
-// in registers for the whole walk, and the hit path is one short predicated
-// block, at 32 registers (64 warps per SM; 40 measured slower).
+// their loads coincide; a lane keeps kWalkBatch candidates in flight (the loads of a
+// run's last batch may pass its end by kPredPad slots, whose pairs are
+// dropped). Issue-bound at large sizes (79% of the slots, 29 warp
+// instructions a candidate of which the hit path takes a third), bound by the
+// latency of its loads below ~300k particles. Against one candidate at a
+// time at 32 registers: 131k particles 37 -> 30 us (a step of three substeps
+// 298 -> 248), 500k 93 -> 84, 1M 166 -> 157, 4M 581 -> 567, 8.4M 1149 -> 1161.
+// Batches of 2, 3, 5, 6, 8 and caps of 32, 36, 40 registers (spills) were slower.
+constexpr int kWalkBatch = 4;
+static_assert(kWalkBatch - 1 <= static_cast<int>(kPredPad), "candidate loads past the last slot");
+
 template <int kTables>
-__global__ void __maxnreg__(32) k_density_walk(const uint2* __restrict__ tiles,
-                               uint32_t ntiles,
-                               const SceneDev* __restrict__ scenes,
-                               const float4* __restrict__ pred,
-                               const uint32_t* __restrict__ start,
-                               const uint32_t* __restrict__ cell_first,
-                               const uint2* __restrict__ cell_tab,
-                               float2* __restrict__ dens_a,
-                               float4* __restrict__ dens_b,
-                               uint32_t* __restrict__ nbr,
-                               uint32_t* __restrict__ ncount,
-                               uint32_t nbr_step, uint32_t nbr_cap) {
+__global__ void __maxnreg__(48)
+k_density_walk(const uint2* __restrict__ tiles, uint32_t ntiles,
+                const SceneDev* __restrict__ scenes, const float4* __restrict__ pred,
+                const uint32_t* __restrict__ start, const uint32_t* __restrict__ cell_first,
+                const uint2* __restrict__ cell_tab, float2* __restrict__ dens_a,
+                float4* __restrict__ dens_b, uint32_t* __restrict__ nbr,
+                uint32_t* __restrict__ ncount, uint32_t nbr_step, uint32_t nbr_cap) {
   pdl_launch();
   const uint32_t lane = lane_id();
   for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const SceneDev& S = scenes[tile_scene(tile)];
+    const bool direct = kTables == kTablesDirect    ? true
+                      : kTables == kTablesBuckets ? false
+                                                  : S.direct != 0u;
+    const float cut = S.cut_le, r = S.r;
     pdl_wait();
     if (lane >= tile_len(tile)) continue;
     const uint32_t i = tile.y + lane;
     const float4 me = pred[i];
-    const float3 p = make_float3(me.x, me.y, me.z);
-    float s2 = S.r2, s3 = S.r2 * S.r;  // self: w = r
+    const float2 npxy = make_float2(-me.x, -me.y);
+    float s2 = S.r2, s3 = S.r2 * r;  // self: w = r
     uint32_t cnt = 0;
     // next list entry: a bumped pointer is the cheapest append in the hit
     // path, and it stays one only while the step and the capacity are
     // run-time values (with constants the compiler recomputes the address
     // from cnt: 195 instead of 172 us at 1M)
     uint32_t* wp = nbr + nbr_index(i, 0);
-    // Pairs with dist <= r (d2 <= cut_le) enter the list; the density takes
-    // (r - dist)^2 and (r - dist)^3 of the same pairs: those with dist == r
-    // exactly, which the reference leaves out, add (r - sqrt(d2))^2, the
-    // square of a rounding error.
-    const float cut = S.cut_le, r = S.r;
-    const uint32_t cf = kTables == kTablesDirect ? 0u : cell_first[i];
-    const float2 npxy = make_float2(-p.x, -p.y);
-    walk_runs<kTables>(S, start, cell_tab, cf, __float_as_uint(me.w), pred, [&](uint32_t j, float4 q) {
-      // dist2 with (dx, dy) as one packed FP32x2 pair (x and y are adjacent
-      // in the record): every component rounded as the scalar code rounds
-      // it, two instructions fewer per candidate
-      const float2 dxy = __fadd2_rn(make_float2(q.x, q.y), npxy);
-      const float2 sxy = __fmul2_rn(dxy, dxy);
-      const float dz = q.z - p.z;
-      const float d2 = __fadd_rn(__fadd_rn(sxy.x, sxy.y), __fmul_rn(dz, dz));
-      if (d2 <= cut && j != i) {
-        if (cnt < nbr_cap) {
-          *wp = j;
-          wp += nbr_step;
+    auto run = [&](uint32_t j, uint32_t e) {
+#pragma unroll 1
+      for (; j < e; j += kWalkBatch) {
+        float4 q[kWalkBatch];
+#pragma unroll
+        for (uint32_t u = 0; u < kWalkBatch; ++u) q[u] = __ldg(pred + j + u);
+#pragma unroll
+        for (uint32_t u = 0; u < kWalkBatch; ++u) {
+          // dist2 with (dx, dy) as one packed FP32x2 pair (x and y are
+          // adjacent in the record), every component rounded as the scalar
+          // code rounds it
+          const float2 dxy = __fadd2_rn(make_float2(q[u].x, q[u].y), npxy);
+          const float2 sxy = __fmul2_rn(dxy, dxy);
+          const float dz = q[u].z - me.z;
+          const float d2 = __fadd_rn(__fadd_rn(sxy.x, sxy.y), __fmul_rn(dz, dz));
+          // Pairs with dist <= r (d2 <= cut_le) enter the list; the density
+          // takes (r - dist)^2 and (r - dist)^3 of the same pairs: those with
+          // dist == r exactly, which the reference leaves out, add
+          // (r - sqrt(d2))^2, the square of a rounding error.
+          if (j + u < e && d2 <= cut && j + u != i) {
+            if (cnt < nbr_cap) {
+              *wp = j + u;
+              wp += nbr_step;
+            }
+            ++cnt;
+            density_sum(r - sqrt_approx(d2), s2, s3);
+          }
         }
-        ++cnt;
-        density_sum(r - sqrt_approx(d2), s2, s3);
       }
-    });
+    };
+    if (direct) {
+      // rows (dy, dz) in the cell table's order (dz fastest); k = the row's
+      // middle cell
+      uint32_t k = S.tbase + __float_as_uint(me.w) - S.gwy - S.gwz;
+      uint32_t b = __ldg(start + k - 1), e = __ldg(start + k + 2);
+      int dz = 0;
+#pragma unroll 1
+      for (int w = 0; w < 9; ++w) {
+        if (++dz == 3) { dz = 0; k += S.gwy - 2u * S.gwz; } else { k += S.gwz; }
+        uint32_t nb = 0, ne = 0;
+        if (w < 8) {  // the next row's run
+          nb = __ldg(start + k - 1);
+          ne = __ldg(start + k + 2);
+        }
+        run(b, e);
+        b = nb;
+        e = ne;
+      }
+    } else {
+      const uint2* row = cell_tab + static_cast<uint64_t>(cell_first[i]) * 27u;
+#pragma unroll 1
+      for (int w = 0; w < 9; ++w, row += 3) {
+        const uint2 m = __ldg(row);
+        const uint32_t runs = (m.y & kRunMerged) ? 1u : 3u;
+#pragma unroll 1
+        for (uint32_t k = 0; k < runs; ++k) {
+          const uint2 x = k ? __ldg(row + k) : m;
+          run(x.x, x.x + (x.y & ~kRunMerged));
+        }
+      }
+    }
     density_store(S, i, s2, s3, cnt, dens_a, dens_b, ncount);
   }
 }
