@@ -234,6 +234,7 @@ int Engine::Init() {
   SPH_CUDA(cudaMemset(d_status_, 0, sizeof(uint32_t)), "cudaMemset");
   SPH_CUDA(cudaMemset(d_out4_, 0, C * sizeof(float4)), "cudaMemset");
   ctx_.scenes = d_scenes_;
+  ctx_.sms = static_cast<uint32_t>(sm_count_);
   ctx_.out4 = d_out4_;
   ctx_.rec_b = reinterpret_cast<float2*>(ctx_.rec_v + C);
   ctx_.status = d_status_;

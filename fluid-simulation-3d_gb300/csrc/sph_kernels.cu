@@ -1834,6 +1834,19 @@ bool coop_form(const LaunchCtx& c, uint32_t ntiles) {
   return c.lanes == 1 && ntiles <= kCoopTiles;
 }
 
+// Launches whose plain neighbour kernels fit the GPU in about one wave (48
+// registers: 40 warps an SM) go out without the programmatic attribute. A
+// kernel started early is placed around its predecessor's resident blocks,
+// and with a single wave that uneven placement stays (more waves even it out):
+// passes of three substeps, us, with it / without: 67k particles 187 / 171, 90k
+// 218 / 180, 130k 245 / 205, 150k 252 / 219, 180k 257 / 252, 195k 266 / 268,
+// 260k 360 / 364; a settled pool of 130k 160 / 142. (The latency forms gain
+// from it: 37k 139 / 141.)
+constexpr uint32_t kWaveWarps = 40;
+bool one_wave(const LaunchCtx& c, uint32_t ntiles) {
+  return ntiles > kRowsTiles && ntiles <= kWaveWarps * c.sms;
+}
+
 cudaError_t launch_sort_reorder(const LaunchCtx& c, const Tiles& old_tiles,
                                 const Tiles& new_tiles, uint32_t total,
                                 cudaStream_t st) {
@@ -1875,7 +1888,7 @@ cudaError_t launch_density(const LaunchCtx& c, const Tiles& tiles,
   const int b = c.block_nbr;
   const uint32_t g = grid_for(tiles.n, b, c.max_blocks);
   if (c.cell_tile <= 1)
-    return launch_pdl(c.pdl,
+    return launch_pdl(c.pdl && !one_wave(c, tiles.n),
                       c.tables == kTablesDirect    ? k_density_walk<kTablesDirect>
                       : c.tables == kTablesBuckets ? k_density_walk<kTablesBuckets>
                                                    : k_density_walk<kTablesMixed>,
@@ -1937,8 +1950,8 @@ cudaError_t launch_pressure(const LaunchCtx& c, const Tiles& tiles,
                                            : pressure_kernel<kTablesMixed>(c.gather, c.lanes);
   // Started early beside k_density_rows' blocks this kernel would run with the
   // L1 their shared memory leaves it (37k particles: 9 us a substep).
-  return launch_pdl(c.pdl && !rows_form(c, tiles.n), kern, grid_for(tiles.n, b, c.max_blocks), b,
-                    st, tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab,
+  return launch_pdl(c.pdl && !rows_form(c, tiles.n) && !one_wave(c, tiles.n), kern,
+                    grid_for(tiles.n, b, c.max_blocks), b, st, tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab,
                     c.dens_a, c.dens_b, c.nbr, c.ncount,
                     c.vel2, c.rec_v, c.rec_b, c.dbg_accp, c.dbg_velp);
 }
@@ -1960,8 +1973,8 @@ cudaError_t launch_visc_integrate(const LaunchCtx& c, const Tiles& tiles,
   auto kern = c.tables == kTablesDirect    ? visc_kernel<kTablesDirect>(c.gather, c.lanes)
               : c.tables == kTablesBuckets ? visc_kernel<kTablesBuckets>(c.gather, c.lanes)
                                            : visc_kernel<kTablesMixed>(c.gather, c.lanes);
-  return launch_pdl(c.pdl, kern, grid_for(tiles.n, b, c.max_blocks), b, st, tiles.d,
-                    tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab, c.nbr,
+  return launch_pdl(c.pdl && !one_wave(c, tiles.n), kern, grid_for(tiles.n, b, c.max_blocks), b,
+                    st, tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab, c.nbr,
                     c.ncount, c.rec_v, c.rec_b, c.pos2, c.vel2,
                     write_out ? c.out4 : nullptr, fuse_next, c.count, c.keyrank,
                     c.dbg_velv, c.status);

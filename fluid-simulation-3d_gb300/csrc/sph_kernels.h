@@ -88,6 +88,7 @@ struct LaunchCtx {
   uint32_t src_limit = 0;  // slots of the layout a substep reads
   bool pdl = true;        // programmatic dependent launch (off while the
                           // engine records phase events between kernels)
+  uint32_t sms = 0;       // multiprocessors of the device
   int block_misc = 256;   // predict/scatter/reorder
   int block_nbr = 128;    // neighbour kernels (density)
   int block_force = 128;  // pressure and viscosity
