@@ -26,6 +26,8 @@
 // uneven sizes.
 #include "sph_kernels.h"
 
+#include <algorithm>
+
 namespace sph {
 
 namespace {
@@ -1834,6 +1836,16 @@ bool coop_form(const LaunchCtx& c, uint32_t ntiles) {
   return c.lanes == 1 && ntiles <= kCoopTiles;
 }
 
+// List entries a lane of the plain force kernels gathers at once: at least 8,
+// then 4, where too few warps hide the loads (the results do not depend on
+// it). Passes of three substeps, us, by 2 / 4 / 8 entries: 32k particles 134 / 124
+// / 120, 37k 137 / 126 / 123, 50k 156 / 146 / 152, 67k 173 / 168 / 171, 90k 178 /
+// 178 / 200.
+constexpr uint32_t kGather8Tiles = 1200;
+int force_gather(const LaunchCtx& c, uint32_t ntiles) {
+  return std::max(c.gather, ntiles <= kGather8Tiles ? 8 : ntiles <= kRowsTiles ? 4 : 2);
+}
+
 // Launches whose plain neighbour kernels fit the GPU in about one wave (48
 // registers: 40 warps an SM) go out without the programmatic attribute. A
 // kernel started early is placed around its predecessor's resident blocks,
@@ -1944,10 +1956,10 @@ cudaError_t launch_pressure(const LaunchCtx& c, const Tiles& tiles,
                       tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab,
                       c.dens_a, c.dens_b, c.nbr, c.ncount, c.vel2, c.rec_v, c.dbg_accp,
                       c.dbg_velp);
-  const int b = c.block_force;
-  auto kern = c.tables == kTablesDirect    ? pressure_kernel<kTablesDirect>(c.gather, c.lanes)
-              : c.tables == kTablesBuckets ? pressure_kernel<kTablesBuckets>(c.gather, c.lanes)
-                                           : pressure_kernel<kTablesMixed>(c.gather, c.lanes);
+  const int b = c.block_force, gather = force_gather(c, tiles.n);
+  auto kern = c.tables == kTablesDirect    ? pressure_kernel<kTablesDirect>(gather, c.lanes)
+              : c.tables == kTablesBuckets ? pressure_kernel<kTablesBuckets>(gather, c.lanes)
+                                           : pressure_kernel<kTablesMixed>(gather, c.lanes);
   // Started early beside k_density_rows' blocks this kernel would run with the
   // L1 their shared memory leaves it (37k particles: 9 us a substep).
   return launch_pdl(c.pdl && !rows_form(c, tiles.n) && !one_wave(c, tiles.n), kern,
@@ -1969,10 +1981,10 @@ cudaError_t launch_visc_integrate(const LaunchCtx& c, const Tiles& tiles,
                       tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab, c.nbr,
                       c.ncount, c.rec_v, c.pos2, c.vel2, write_out ? c.out4 : nullptr, fuse_next,
                       c.count, c.keyrank, c.dbg_velv, c.status);
-  const int b = c.block_force;
-  auto kern = c.tables == kTablesDirect    ? visc_kernel<kTablesDirect>(c.gather, c.lanes)
-              : c.tables == kTablesBuckets ? visc_kernel<kTablesBuckets>(c.gather, c.lanes)
-                                           : visc_kernel<kTablesMixed>(c.gather, c.lanes);
+  const int b = c.block_force, gather = force_gather(c, tiles.n);
+  auto kern = c.tables == kTablesDirect    ? visc_kernel<kTablesDirect>(gather, c.lanes)
+              : c.tables == kTablesBuckets ? visc_kernel<kTablesBuckets>(gather, c.lanes)
+                                           : visc_kernel<kTablesMixed>(gather, c.lanes);
   return launch_pdl(c.pdl && !one_wave(c, tiles.n), kern, grid_for(tiles.n, b, c.max_blocks), b,
                     st, tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab, c.nbr,
                     c.ncount, c.rec_v, c.rec_b, c.pos2, c.vel2,

@@ -75,7 +75,9 @@ typedef struct sph_tuning {
                          particle, each summing every other neighbour of
                          its list; agrees with 32 to rounding)            */
   int32_t gather;     /* neighbour-list entries whose gathers the force
-                         kernels issue together: 2, 3, 4 or 8 (default 2) */
+                         kernels issue together: 2, 3, 4 or 8 (default 2;
+                         small launches issue 4 or 8 at least). Results do
+                         not depend on it                                 */
   int32_t force_block; /* threads per block of the pressure and viscosity
                           kernels (multiple of 32, 32..1024); 0 = block   */
   int32_t table;      /* key table of the sort: 0 = one entry per cell of
