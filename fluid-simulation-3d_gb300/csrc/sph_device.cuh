@@ -87,6 +87,8 @@ struct SceneDev {
   float ndamp;        // -1 * dampFactor                    (:94)
   float pdt;          // prediction look-ahead 1/120        (:47)
   float dt;           // substep dt
+  uint32_t tile0;     // tiles of the scenes before this one
+  uint32_t old_base;  // first slot in the layout the next sort reads
 };
 
 // x % d for 32-bit x, d >= 1, with M = floor((2^64-1)/d) + 1 (Lemire et al.,

@@ -243,6 +243,25 @@ __device__ __forceinline__ void walk_runs(const SceneDev& S,
   }
 }
 
+// ------------------------------------------------------------------- tiles
+// Tile tables after a change of the layout, a thread a tile: its scene is the
+// last one whose first tile is not past it (a scene without particles shares
+// its first tile with the next). 16 B a tile, so bound by the launch.
+__global__ void k_tiles(const SceneDev* __restrict__ scene_table, uint32_t scenes, uint32_t ntiles,
+                        uint2* __restrict__ tiles_old, uint2* __restrict__ tiles_new) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= ntiles) return;
+  uint32_t lo = 0, hi = scenes;  // tile0 of lo is <= t, of hi (if any) > t
+  while (hi - lo > 1u) {
+    const uint32_t mid = lo + (hi - lo) / 2u;
+    if (scene_table[mid].tile0 <= t) lo = mid; else hi = mid;
+  }
+  const SceneDev& S = scene_table[lo];
+  const uint32_t f = (t - S.tile0) * kTile, len = min(static_cast<uint32_t>(kTile), S.n - f);
+  tiles_old[t] = make_tile(lo, S.old_base + f, len);
+  tiles_new[t] = make_tile(lo, S.base + f, len);
+}
+
 // ----------------------------------------------------------------- predict
 __device__ __forceinline__ void predict_key(const SceneDev& S, float4 p,
                                             float4 v, uint32_t& key,
@@ -1785,6 +1804,13 @@ template <class... KArgs, class... Args>
 cudaError_t launch_pdl(bool pdl, void (*kernel)(KArgs...), uint32_t grid, int block,
                        cudaStream_t st, Args... args) {
   return launch_pdl_smem(pdl, kernel, grid, block, 0, st, args...);
+}
+
+cudaError_t launch_tiles(const SceneDev* scene_table, uint32_t scenes, uint32_t ntiles,
+                         uint2* tiles_old, uint2* tiles_new, cudaStream_t st) {
+  if (ntiles == 0) return cudaSuccess;
+  k_tiles<<<(ntiles + 255) / 256, 256, 0, st>>>(scene_table, scenes, ntiles, tiles_old, tiles_new);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_predict_hash(const LaunchCtx& c, const Tiles& old_tiles,

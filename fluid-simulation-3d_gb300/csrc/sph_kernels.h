@@ -104,6 +104,10 @@ inline uint32_t grid_for(uint32_t ntiles, int block, uint32_t max_blocks) {
 
 uint32_t scan_partials_needed(uint64_t len);
 
+// Tile tables of the layout the next sort reads and the one it writes, from
+// the device's scene table (`scenes` entries, ascending tile0).
+cudaError_t launch_tiles(const SceneDev* scene_table, uint32_t scenes, uint32_t ntiles,
+                         uint2* tiles_old, uint2* tiles_new, cudaStream_t st);
 cudaError_t launch_predict_hash(const LaunchCtx& c, const Tiles& old_tiles,
                                 cudaStream_t st);
 cudaError_t launch_scan(const LaunchCtx& c, uint32_t len, cudaStream_t st);
