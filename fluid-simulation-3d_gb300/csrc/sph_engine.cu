@@ -77,6 +77,8 @@ uint32_t GridAxis(float h, float r, uint32_t* origin) {
 constexpr uint64_t kDirectCellsPerParticle = 4;
 constexpr uint64_t kTablePerParticle = kDirectCellsPerParticle;
 constexpr uint64_t kTableAllowance = 65536;
+static_assert(kTablePerParticle % 4 == 0 && kTableAllowance % 4 == 0,
+              "k_clear zeroes the histogram in words of four entries");
 
 // The scene's constants with a bucket table at `tbase`; the caller switches
 // to a direct table (direct = 1) where it has room for one.
@@ -392,12 +394,9 @@ int Engine::Load(uint32_t id, const float* pos3, const float* vel3,
                        uploaded_substeps_ > 0 && !layout_dirty_ &&
                        n_tiles_old_ == n_tiles_new_ && total_ == n;
   if (rows) {
-    if (predict && count_extent_)
-      SPH_CUDA(cudaMemsetAsync(ctx_.count, 0, sizeof(uint32_t) * count_extent_, st),
-               "histogram reset");
     SPH_CUDA(launch_import_rows(old_base_[id], n, rp, rv, d_pos_[cur_], d_vel_[cur_],
                                 ctx_.dens_a, predict ? ctx_.scenes + id : nullptr, ctx_.count,
-                                ctx_.keyrank, st),
+                                predict ? count_extent_ : 0u, ctx_.keyrank, st),
              "import kernel");
     if (predict) {
       carry_valid_ = true;

@@ -161,10 +161,11 @@ cudaError_t launch_import(uint32_t first, uint32_t n, const float* ipos,
 // The same import for 16-byte aligned rows the device addresses directly (its
 // own memory or pinned host buffers): rows move as aligned float4 per warp.
 // With `scene` (the scene's device constants) it also writes the next step's
-// first prediction (keyrank, histogram in count) as k_predict_hash does.
+// first prediction (keyrank, histogram in count, whose first `clear` entries
+// hold an unused one) as k_predict_hash does.
 cudaError_t launch_import_rows(uint32_t first, uint32_t n, const float* ipos,
                                const float* ivel, float4* pos, float4* vel, float2* dens,
-                               const SceneDev* scene, uint32_t* count, uint4* keyrank,
-                               cudaStream_t st);
+                               const SceneDev* scene, uint32_t* count, uint32_t clear,
+                               uint4* keyrank, cudaStream_t st);
 
 }  // namespace sph
