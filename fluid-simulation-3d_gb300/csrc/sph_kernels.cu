@@ -1321,7 +1321,7 @@ __device__ __forceinline__ void integrate(const SceneDev& S, const SceneDev& S_n
 
 // kLanes lanes per particle as in k_pressure.
 template <int kGather, int kTables, int kLanes>
-__global__ void k_visc_integrate(
+__device__ __forceinline__ void visc_tiles(
     const uint2* __restrict__ tiles, uint32_t ntiles,
     const SceneDev* __restrict__ scenes, const float4* __restrict__ pred,
     const uint32_t* __restrict__ start,
@@ -1396,6 +1396,40 @@ __global__ void k_visc_integrate(
       if (__any_sync(kFull, bad) && lane == 0) flag(status, kStatusNonFinite);
     }
   }
+}
+
+template <int kGather, int kTables, int kLanes>
+__global__ void k_visc_integrate(
+    const uint2* __restrict__ tiles, uint32_t ntiles,
+    const SceneDev* __restrict__ scenes, const float4* __restrict__ pred,
+    const uint32_t* __restrict__ start,
+    const uint32_t* __restrict__ cell_first, const uint2* __restrict__ cell_tab,
+    const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ ncount, const float4* __restrict__ rec_v,
+    const float2* __restrict__ rec_b,
+    float4* __restrict__ pos, float4* __restrict__ vel,
+    float4* __restrict__ out4, int fuse_next, uint32_t* __restrict__ count,
+    uint4* __restrict__ keyrank, float4* __restrict__ dbg_velv,
+    uint32_t* status) {
+  visc_tiles<kGather, kTables, kLanes>(tiles, ntiles, scenes, pred, start, cell_first, cell_tab, nbr, ncount, rec_v,
+                                       rec_b, pos, vel, out4, fuse_next, count, keyrank, dbg_velv, status);
+}
+
+// The default form for launches of many waves (dense_form): 40 registers, 48
+// instead of 40 warps an SM, at 16 B of spills outside the loop.
+template <int kTables>
+__global__ void __maxnreg__(40) k_visc_dense(
+    const uint2* __restrict__ tiles, uint32_t ntiles,
+    const SceneDev* __restrict__ scenes, const float4* __restrict__ pred,
+    const uint32_t* __restrict__ start,
+    const uint32_t* __restrict__ cell_first, const uint2* __restrict__ cell_tab,
+    const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ ncount, const float4* __restrict__ rec_v,
+    const float2* __restrict__ rec_b,
+    float4* __restrict__ pos, float4* __restrict__ vel,
+    float4* __restrict__ out4, int fuse_next, uint32_t* __restrict__ count,
+    uint4* __restrict__ keyrank, float4* __restrict__ dbg_velv,
+    uint32_t* status) {
+  visc_tiles<2, kTables, 1>(tiles, ntiles, scenes, pred, start, cell_first, cell_tab, nbr, ncount, rec_v,
+                            rec_b, pos, vel, out4, fuse_next, count, keyrank, dbg_velv, status);
 }
 
 // Latency form for small launches, as k_pressure_coop: the terms of visc_pair
@@ -1904,6 +1938,16 @@ bool one_wave(const LaunchCtx& c, uint32_t ntiles) {
   return ntiles > kRowsTiles && ntiles <= kWaveWarps * c.sms;
 }
 
+// Launches whose viscosity pass runs at 48 instead of 40 warps an SM: more than
+// three waves of the latter (with fewer, the last wave costs more than the
+// occupancy gives). Viscosity per substep, us, 40 / 48 warps: 262k particles 28.7
+// / 30.2, 500k 43.6 / 45.9, 700k 57.8 / 54.5, 1M 82.2 / 79.1 (a settled pool
+// 54.0 / 52.3), 2M 149.7 / 140.3, 8.4M 583 / 539. The pressure pass needs 48
+// registers: at 40 it spills in its loop (1M 91 / 104).
+bool dense_form(const LaunchCtx& c, uint32_t ntiles) {
+  return c.lanes == 1 && c.gather == 2 && ntiles > 3u * kWaveWarps * c.sms;
+}
+
 cudaError_t launch_sort_reorder(const LaunchCtx& c, const Tiles& old_tiles,
                                 const Tiles& new_tiles, uint32_t total,
                                 cudaStream_t st) {
@@ -2027,7 +2071,10 @@ cudaError_t launch_visc_integrate(const LaunchCtx& c, const Tiles& tiles,
                       c.ncount, c.rec_v, c.pos2, c.vel2, write_out ? c.out4 : nullptr, fuse_next,
                       c.count, c.keyrank, c.dbg_velv, c.status);
   const int b = c.block_force, gather = force_gather(c, tiles.n);
-  auto kern = c.tables == kTablesDirect    ? visc_kernel<kTablesDirect>(gather, c.lanes)
+  auto kern = dense_form(c, tiles.n) ? (c.tables == kTablesDirect    ? k_visc_dense<kTablesDirect>
+                                        : c.tables == kTablesBuckets ? k_visc_dense<kTablesBuckets>
+                                                                     : k_visc_dense<kTablesMixed>)
+              : c.tables == kTablesDirect  ? visc_kernel<kTablesDirect>(gather, c.lanes)
               : c.tables == kTablesBuckets ? visc_kernel<kTablesBuckets>(gather, c.lanes)
                                            : visc_kernel<kTablesMixed>(gather, c.lanes);
   return launch_pdl(c.pdl && !one_wave(c, tiles.n), kern, grid_for(tiles.n, b, c.max_blocks), b,
