@@ -147,9 +147,6 @@ Engine::~Engine() {
     if (e) cudaEventDestroy(e);
   if (join_in_) cudaEventDestroy(join_in_);
   if (join_out_) cudaEventDestroy(join_out_);
-  if (staged_) cudaEventSynchronize(staged_done_);
-  if (staged_done_) cudaEventDestroy(staged_done_);
-  if (h_scenes_) cudaFreeHost(h_scenes_);
   if (work_) cudaStreamDestroy(work_);
   void* ptrs[] = {d_scenes_, d_tiles_old_, d_tiles_new_, d_pos_[0], d_pos_[1],
                   d_vel_[0], d_vel_[1], ctx_.pred, ctx_.rec_v, ctx_.dens_a,
@@ -198,10 +195,6 @@ int Engine::Init() {
            "cudaEventCreate");
   SPH_CUDA(cudaEventCreateWithFlags(&join_out_, cudaEventDisableTiming),
            "cudaEventCreate");
-  SPH_CUDA(cudaEventCreateWithFlags(&staged_done_, cudaEventDisableTiming),
-           "cudaEventCreate");
-  int rc = StageScenes(1);
-  if (rc != SPH_OK) return rc;
   const uint64_t C = capacity_;
   const uint64_t max_tiles = C / kTile + max_scenes_ + 1;
   cudaError_t e = cudaSuccess;
@@ -446,8 +439,8 @@ int Engine::BuildLayout(cudaStream_t st) {
   return SPH_OK;
 }
 
-// A changed layout or scene table cannot become part of a caller's graph (its
-// staging buffer is rewritten by the next change): the wait fails the call
+// A changed layout or scene table cannot become part of a caller's graph (a
+// replay would bring back what later calls changed): the wait fails the call
 // and the capture, as a stream that is being captured cannot be waited for.
 int Engine::RefuseCapture(cudaStream_t st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -457,25 +450,9 @@ int Engine::RefuseCapture(cudaStream_t st) {
   return SPH_OK;
 }
 
-// The pinned staging of the scene table, for at least `count` scenes, free to
-// be rewritten (the copy that last read it has finished).
-int Engine::StageScenes(uint32_t count) {
-  if (staged_) SPH_CUDA(cudaEventSynchronize(staged_done_), "cudaEventSynchronize");
-  staged_ = false;
-  if (count <= stage_cap_) return SPH_OK;
-  if (h_scenes_) cudaFreeHost(h_scenes_);
-  h_scenes_ = nullptr;
-  stage_cap_ = 0;
-  const uint32_t cap = std::min(max_scenes_, std::max(count, kStageScenes));
-  SPH_CUDA(cudaMallocHost(reinterpret_cast<void**>(&h_scenes_), sizeof(SceneDev) * cap),
-           "cudaMallocHost");
-  stage_cap_ = cap;
-  return SPH_OK;
-}
-
 int Engine::UploadScenes(int substeps, cudaStream_t st) {
   if (!scenes_dirty_ && uploaded_substeps_ == substeps) return SPH_OK;
-  int rc = RefuseCapture(st);
+  const int rc = RefuseCapture(st);
   if (rc != SPH_OK) return rc;
   std::vector<SceneDev> h(max_scenes_);
   uint32_t hi = 0, tile = 0;
@@ -514,22 +491,15 @@ int Engine::UploadScenes(int substeps, cudaStream_t st) {
     tables_ = tables;
     ReleaseGraphs();
   }
-  // Pinned staging and tile tables written by a kernel: filling the tables on
-  // the host, copying them from pageable memory and waiting for the copies
-  // held a new scene's first step up by 0.2 ms at 1M particles (its call 258
-  // -> 57 us) and 1.3 ms at 8.4M.
-  if (hi) {
-    rc = StageScenes(hi);
-    if (rc != SPH_OK) return rc;
-    std::copy(h.begin(), h.begin() + hi, h_scenes_);
-    SPH_CUDA(cudaMemcpyAsync(d_scenes_, h_scenes_, sizeof(SceneDev) * hi,
-                             cudaMemcpyHostToDevice, st), "upload scenes");
-    SPH_CUDA(cudaEventRecord(staged_done_, st), "cudaEventRecord");
-    staged_ = true;
-    if (layout_dirty_)
-      SPH_CUDA(launch_tiles(d_scenes_, hi, n_tiles_new_, d_tiles_old_, d_tiles_new_, st),
-               "tile tables");
-  }
+  // The scene table travels as kernel parameters and a kernel writes the tile
+  // tables: filling those on the host, copying both from pageable memory and
+  // waiting for the copies held a new scene's first step up by 0.2 ms at 1M
+  // particles (its call 258 -> 57 us) and 1.3 ms at 8.4M. (Pinned staging is as
+  // fast but costs 0.13 ms when a handle is made and 0.19 when it is freed.)
+  SPH_CUDA(launch_scenes(d_scenes_, h.data(), hi, st), "upload scenes");
+  if (layout_dirty_)
+    SPH_CUDA(launch_tiles(d_scenes_, hi, n_tiles_new_, d_tiles_old_, d_tiles_new_, st),
+             "tile tables");
   scene_dev_ = std::move(h);
   scenes_dirty_ = false;
   uploaded_substeps_ = substeps;

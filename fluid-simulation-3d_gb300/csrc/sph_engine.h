@@ -103,7 +103,6 @@ class Engine {
   int UploadScenes(int substeps, cudaStream_t st);
   int RunSubsteps(int substeps, cudaStream_t st, bool carry);
   int RefuseCapture(cudaStream_t st);
-  int StageScenes(uint32_t count);
   void ReleaseGraphs();
 
   uint64_t capacity_;
@@ -133,13 +132,6 @@ class Engine {
 
   // device memory
   SceneDev* d_scenes_ = nullptr;
-  // pinned staging of the scene table (grown beyond kStageScenes on demand);
-  // staged_done_ follows the copy that last read it (staged_: there is one)
-  static constexpr uint32_t kStageScenes = 256;
-  SceneDev* h_scenes_ = nullptr;
-  uint32_t stage_cap_ = 0;
-  bool staged_ = false;
-  cudaEvent_t staged_done_ = nullptr;
   uint2* d_tiles_old_ = nullptr;
   uint2* d_tiles_new_ = nullptr;
   uint32_t n_tiles_old_ = 0, n_tiles_new_ = 0;

@@ -243,12 +243,30 @@ __device__ __forceinline__ void walk_runs(const SceneDev& S,
   }
 }
 
-// ------------------------------------------------------------------- tiles
+// --------------------------------------------------------- scenes and tiles
+// Part of the scene table as a kernel parameter (up to the parameters' 4 KB,
+// and 32 KB for large batches): it needs no staging memory and no wait, and is
+// copied when the launch is made.
+template <int N> struct SceneChunk {
+  SceneDev s[N];
+};
+constexpr int kFewScenes = 4000 / sizeof(SceneDev);
+constexpr int kManyScenes = 32000 / sizeof(SceneDev);
+
+template <int N>
+__global__ void k_scenes(const __grid_constant__ SceneChunk<N> chunk, uint32_t words,
+                         uint32_t* __restrict__ table) {
+  pdl_launch();
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(&chunk);
+  for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) table[i] = w[i];
+}
+
 // Tile tables after a change of the layout, a thread a tile: its scene is the
 // last one whose first tile is not past it (a scene without particles shares
 // its first tile with the next). 16 B a tile, so bound by the launch.
 __global__ void k_tiles(const SceneDev* __restrict__ scene_table, uint32_t scenes, uint32_t ntiles,
                         uint2* __restrict__ tiles_old, uint2* __restrict__ tiles_new) {
+  pdl_wait();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ntiles) return;
   uint32_t lo = 0, hi = scenes;  // tile0 of lo is <= t, of hi (if any) > t
@@ -1859,11 +1877,34 @@ cudaError_t launch_pdl(bool pdl, void (*kernel)(KArgs...), uint32_t grid, int bl
   return launch_pdl_smem(pdl, kernel, grid, block, 0, st, args...);
 }
 
+template <int N>
+cudaError_t launch_scene_chunk(SceneDev* table, const SceneDev* host, uint32_t count,
+                               cudaStream_t st) {
+  SceneChunk<N> chunk;
+  std::copy(host, host + count, chunk.s);
+  k_scenes<N><<<1, 256, 0, st>>>(chunk, count * static_cast<uint32_t>(sizeof(SceneDev) / 4),
+                                 reinterpret_cast<uint32_t*>(table));
+  return cudaGetLastError();
+}
+
+cudaError_t launch_scenes(SceneDev* scene_table, const SceneDev* host, uint32_t scenes,
+                          cudaStream_t st) {
+  cudaError_t e = cudaSuccess;
+  for (uint32_t s = 0; s < scenes && e == cudaSuccess;) {
+    const uint32_t left = scenes - s;
+    const uint32_t n = std::min<uint32_t>(left, left <= kFewScenes ? kFewScenes : kManyScenes);
+    e = left <= kFewScenes ? launch_scene_chunk<kFewScenes>(scene_table + s, host + s, n, st)
+                           : launch_scene_chunk<kManyScenes>(scene_table + s, host + s, n, st);
+    s += n;
+  }
+  return e;
+}
+
 cudaError_t launch_tiles(const SceneDev* scene_table, uint32_t scenes, uint32_t ntiles,
                          uint2* tiles_old, uint2* tiles_new, cudaStream_t st) {
   if (ntiles == 0) return cudaSuccess;
-  k_tiles<<<(ntiles + 255) / 256, 256, 0, st>>>(scene_table, scenes, ntiles, tiles_old, tiles_new);
-  return cudaGetLastError();
+  return launch_pdl(true, k_tiles, (ntiles + 255) / 256, 256, st, scene_table, scenes, ntiles,
+                    tiles_old, tiles_new);
 }
 
 cudaError_t launch_predict_hash(const LaunchCtx& c, const Tiles& old_tiles,

@@ -104,6 +104,10 @@ inline uint32_t grid_for(uint32_t ntiles, int block, uint32_t max_blocks) {
 
 uint32_t scan_partials_needed(uint64_t len);
 
+// The host's scene table to the device (copied into the launches before the
+// call returns).
+cudaError_t launch_scenes(SceneDev* scene_table, const SceneDev* host, uint32_t scenes,
+                          cudaStream_t st);
 // Tile tables of the layout the next sort reads and the one it writes, from
 // the device's scene table (`scenes` entries, ascending tile0).
 cudaError_t launch_tiles(const SceneDev* scene_table, uint32_t scenes, uint32_t ntiles,

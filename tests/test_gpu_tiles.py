@@ -1,6 +1,6 @@
 """The tile tables a layout change writes on the device: scenes of sizes around
 a tile's 32 slots, with removed scenes between live ones and more scenes than
-the staging buffer's first size, step bit for bit as each does alone."""
+one launch's parameters hold, step bit for bit as each does alone."""
 import numpy as np
 import pytest
 
