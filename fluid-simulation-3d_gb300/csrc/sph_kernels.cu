@@ -713,8 +713,8 @@ __device__ __forceinline__ void density_store(const SceneDev& S, uint32_t i,
 constexpr int kWalkBatch = 4;
 static_assert(kWalkBatch - 1 <= static_cast<int>(kPredPad), "candidate loads past the last slot");
 
-template <int kTables>
-__global__ void __maxnreg__(48)
+template <int kTables, int kRegs>
+__global__ void __maxnreg__(kRegs)
 k_density_walk(const uint2* __restrict__ tiles, uint32_t ntiles,
                 const SceneDev* __restrict__ scenes, const float4* __restrict__ pred,
                 const uint32_t* __restrict__ start, const uint32_t* __restrict__ cell_first,
@@ -1956,16 +1956,6 @@ bool coop_form(const LaunchCtx& c, uint32_t ntiles) {
   return c.lanes == 1 && ntiles <= kCoopTiles;
 }
 
-// List entries a lane of the plain force kernels gathers at once: at least 8,
-// then 4, where too few warps hide the loads (the results do not depend on
-// it). Passes of three substeps, us, by 2 / 4 / 8 entries: 32k particles 134 / 124
-// / 120, 37k 137 / 126 / 123, 50k 156 / 146 / 152, 67k 173 / 168 / 171, 90k 178 /
-// 178 / 200.
-constexpr uint32_t kGather8Tiles = 1200;
-int force_gather(const LaunchCtx& c, uint32_t ntiles) {
-  return std::max(c.gather, ntiles <= kGather8Tiles ? 8 : ntiles <= kRowsTiles ? 4 : 2);
-}
-
 // Launches whose plain neighbour kernels fit the GPU in about one wave (48
 // registers: 40 warps an SM) go out without the programmatic attribute. A
 // kernel started early is placed around its predecessor's resident blocks,
@@ -1974,19 +1964,42 @@ int force_gather(const LaunchCtx& c, uint32_t ntiles) {
 // 218 / 180, 130k 245 / 205, 150k 252 / 219, 180k 257 / 252, 195k 266 / 268,
 // 260k 360 / 364; a settled pool of 130k 160 / 142. (The latency forms gain
 // from it: 37k 139 / 141.)
+//
+// Between 40 and 48 warps an SM the density and viscosity passes run at 40
+// registers (some spills), which keeps them to one wave; the pressure pass
+// would spill in its loop and stays at 48. Passes of three substeps, us, two
+// waves / one: 200k particles 279 / 278, 210k 313 / 295, 220k 328 / 302, 232k 342
+// / 315; a settled pool of 220k 207 / 199.
 constexpr uint32_t kWaveWarps = 40;
+constexpr uint32_t kDenseWarps = 48;  // at 40 registers
+bool dense_wave(const LaunchCtx& c, uint32_t ntiles) {
+  return c.lanes == 1 && c.gather == 2 && c.cell_tile <= 1 && ntiles > kWaveWarps * c.sms &&
+         ntiles <= kDenseWarps * c.sms;
+}
 bool one_wave(const LaunchCtx& c, uint32_t ntiles) {
-  return ntiles > kRowsTiles && ntiles <= kWaveWarps * c.sms;
+  return ntiles > kRowsTiles && (ntiles <= kWaveWarps * c.sms || dense_wave(c, ntiles));
 }
 
-// Launches whose viscosity pass runs at 48 instead of 40 warps an SM: more than
-// three waves of the latter (with fewer, the last wave costs more than the
-// occupancy gives). Viscosity per substep, us, 40 / 48 warps: 262k particles 28.7
-// / 30.2, 500k 43.6 / 45.9, 700k 57.8 / 54.5, 1M 82.2 / 79.1 (a settled pool
-// 54.0 / 52.3), 2M 149.7 / 140.3, 8.4M 583 / 539. The pressure pass needs 48
-// registers: at 40 it spills in its loop (1M 91 / 104).
+// Launches whose viscosity pass runs at 48 instead of 40 warps an SM: those
+// and the ones of more than three waves of the latter (between them the last
+// wave costs more than the occupancy gives). Viscosity per substep, us, 40 / 48
+// warps: 262k particles 28.7 / 30.2, 500k 43.6 / 45.9, 700k 57.8 / 54.5, 1M 82.2 /
+// 79.1 (a settled pool 54.0 / 52.3), 2M 149.7 / 140.3, 8.4M 583 / 539. The pressure
+// pass needs 48 registers: at 40 it spills in its loop (1M 91 / 104).
+constexpr uint32_t kDenseWaves = 3;
 bool dense_form(const LaunchCtx& c, uint32_t ntiles) {
-  return c.lanes == 1 && c.gather == 2 && ntiles > 3u * kWaveWarps * c.sms;
+  return dense_wave(c, ntiles) ||
+         (c.lanes == 1 && c.gather == 2 && ntiles > kDenseWaves * kWaveWarps * c.sms);
+}
+
+// List entries a lane of the plain force kernels gathers at once: at least 8,
+// then 4, where too few warps hide the loads (the results do not depend on
+// it). Passes of three substeps, us, by 2 / 4 / 8 entries: 32k particles 134 / 124
+// / 120, 37k 137 / 126 / 123, 50k 156 / 146 / 152, 67k 173 / 168 / 171, 90k 178 /
+// 178 / 200.
+constexpr uint32_t kGather8Tiles = 1200;
+int force_gather(const LaunchCtx& c, uint32_t ntiles) {
+  return std::max(c.gather, ntiles <= kGather8Tiles ? 8 : ntiles <= kRowsTiles ? 4 : 2);
 }
 
 cudaError_t launch_sort_reorder(const LaunchCtx& c, const Tiles& old_tiles,
@@ -2017,6 +2030,12 @@ cudaError_t launch_sort_reorder(const LaunchCtx& c, const Tiles& old_tiles,
   return e;
 }
 
+template <int kRegs> auto density_kernel(int tables) {
+  return tables == kTablesDirect    ? k_density_walk<kTablesDirect, kRegs>
+         : tables == kTablesBuckets ? k_density_walk<kTablesBuckets, kRegs>
+                                    : k_density_walk<kTablesMixed, kRegs>;
+}
+
 cudaError_t launch_density(const LaunchCtx& c, const Tiles& tiles,
                            cudaStream_t st) {
   if (tiles.n == 0) return cudaSuccess;
@@ -2031,9 +2050,8 @@ cudaError_t launch_density(const LaunchCtx& c, const Tiles& tiles,
   const uint32_t g = grid_for(tiles.n, b, c.max_blocks);
   if (c.cell_tile <= 1)
     return launch_pdl(c.pdl && !one_wave(c, tiles.n),
-                      c.tables == kTablesDirect    ? k_density_walk<kTablesDirect>
-                      : c.tables == kTablesBuckets ? k_density_walk<kTablesBuckets>
-                                                   : k_density_walk<kTablesMixed>,
+                      dense_wave(c, tiles.n) ? density_kernel<40>(c.tables)
+                                             : density_kernel<48>(c.tables),
                       g, b, st, tiles.d, tiles.n, c.scenes, c.pred,
                       c.start, c.cell_first, c.cell_tab, c.dens_a, c.dens_b, c.nbr,
                       c.ncount, 32u, kNbrCap);

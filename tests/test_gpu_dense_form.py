@@ -1,7 +1,8 @@
 """Launches of many waves run the viscosity pass at more warps an SM (another
-register cap, the same code): scenes in a batch beside a filler of 600k
-particles step bit for bit as alone, where the launch is small. Clouds from a
-lone particle to lists that overflow, under each form of the key tables."""
+register cap, the same code), those of a little more than one wave also the
+density pass: scenes in a batch beside a filler of such a size step bit for bit as alone, where the
+launch is small. Clouds from a lone particle to lists that overflow, under each
+form of the key tables."""
 import numpy as np
 import pytest
 
@@ -9,18 +10,20 @@ from test_gpu_latency_forms import cloud
 
 pytestmark = pytest.mark.gpu
 
-FILLER = 600000  # particles: more than three waves of 40 warps an SM
+# particles: between 40 and 48 warps an SM; more than three of 40
+FILLERS = [205000, 600000]
 
 
+@pytest.mark.parametrize("fill", FILLERS)
 @pytest.mark.parametrize("table", [0, 1, 2])
-def test_large_launch_equals_alone(gpu_lib, table):
+def test_large_launch_equals_alone(gpu_lib, table, fill):
     import fluidsim
     from fluidsim import scenes
     dt = 1.0 / 240.0
     scs = [cloud(n, side, 7 + n) for n, side in [(1, 1.0), (33, 1.0), (1500, 0.9), (4097, 3.6)]]
-    pos, vel, bound = scenes.fill_box_scene(np.random.default_rng(5), FILLER, 0.5, (1.0, 1.0, 1.0))
+    pos, vel, bound = scenes.fill_box_scene(np.random.default_rng(5), fill, 0.5, (1.0, 1.0, 1.0))
     filler = scenes.SimParams(radius=0.35, bound=bound, **scenes.DAM_CONSTANTS)
-    b = fluidsim.Batch(FILLER + sum(s[1].shape[0] for s in scs), len(scs) + 1)
+    b = fluidsim.Batch(fill + sum(s[1].shape[0] for s in scs), len(scs) + 1)
     b.set_tuning(table=table)
     b.add(filler, pos, vel, dt)
     ids = [b.add(*s, dt) for s in scs]
