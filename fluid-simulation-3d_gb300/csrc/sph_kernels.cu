@@ -1996,10 +1996,17 @@ bool dense_form(const LaunchCtx& c, uint32_t ntiles) {
 // then 4, where too few warps hide the loads (the results do not depend on
 // it). Passes of three substeps, us, by 2 / 4 / 8 entries: 32k particles 134 / 124
 // / 120, 37k 137 / 126 / 123, 50k 156 / 146 / 152, 67k 173 / 168 / 171, 90k 178 /
-// 178 / 200.
+// 178 / 200. Three, at 59 registers and 32 warps an SM, where those make no more
+// waves than the 40 warps of two: 236k 346 / 335 (two / three entries), 284k 375 /
+// 361, 308k 387 / 375, 428k 517 / 504; settled pools 215 / 211, 229 / 227, 239 /
+// 237, 317 / 314; but 332k 405 / 410, 380k 441 / 462, 500k 565 / 565.
 constexpr uint32_t kGather8Tiles = 1200;
+constexpr uint32_t kGather3Warps = 32;
 int force_gather(const LaunchCtx& c, uint32_t ntiles) {
-  return std::max(c.gather, ntiles <= kGather8Tiles ? 8 : ntiles <= kRowsTiles ? 4 : 2);
+  const auto waves = [&](uint32_t warps) { return (ntiles + warps * c.sms - 1) / (warps * c.sms); };
+  const bool three = c.lanes == 1 && ntiles > kDenseWarps * c.sms && ntiles <= kDenseWaves * kWaveWarps * c.sms &&
+                     waves(kGather3Warps) == waves(kWaveWarps);
+  return std::max(c.gather, ntiles <= kGather8Tiles ? 8 : ntiles <= kRowsTiles ? 4 : three ? 3 : 2);
 }
 
 cudaError_t launch_sort_reorder(const LaunchCtx& c, const Tiles& old_tiles,

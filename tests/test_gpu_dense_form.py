@@ -1,6 +1,7 @@
 """Launches of many waves run the viscosity pass at more warps an SM (another
 register cap, the same code), those of a little more than one wave also the
-density pass: scenes in a batch beside a filler of such a size step bit for bit as alone, where the
+density pass, and some of a few waves gather three list entries at once: scenes
+in a batch beside a filler of such a size step bit for bit as alone, where the
 launch is small. Clouds from a lone particle to lists that overflow, under each
 form of the key tables."""
 import numpy as np
@@ -10,8 +11,8 @@ from test_gpu_latency_forms import cloud
 
 pytestmark = pytest.mark.gpu
 
-# particles: between 40 and 48 warps an SM; more than three of 40
-FILLERS = [205000, 600000]
+# particles: between 40 and 48 warps an SM; two waves of 32; more than three of 40
+FILLERS = [205000, 250000, 600000]
 
 
 @pytest.mark.parametrize("fill", FILLERS)
