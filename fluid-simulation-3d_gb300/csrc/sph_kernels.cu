@@ -1972,6 +1972,9 @@ bool coop_form(const LaunchCtx& c, uint32_t ntiles) {
 // / 315; a settled pool of 220k 207 / 199.
 constexpr uint32_t kWaveWarps = 40;
 constexpr uint32_t kDenseWarps = 48;  // at 40 registers
+uint32_t waves(const LaunchCtx& c, uint32_t ntiles, uint32_t warps) {
+  return (ntiles + warps * c.sms - 1) / (warps * c.sms);
+}
 bool dense_wave(const LaunchCtx& c, uint32_t ntiles) {
   return c.lanes == 1 && c.gather == 2 && c.cell_tile <= 1 && ntiles > kWaveWarps * c.sms &&
          ntiles <= kDenseWarps * c.sms;
@@ -1980,16 +1983,18 @@ bool one_wave(const LaunchCtx& c, uint32_t ntiles) {
   return ntiles > kRowsTiles && (ntiles <= kWaveWarps * c.sms || dense_wave(c, ntiles));
 }
 
-// Launches whose viscosity pass runs at 48 instead of 40 warps an SM: those
-// and the ones of more than three waves of the latter (between them the last
-// wave costs more than the occupancy gives). Viscosity per substep, us, 40 / 48
-// warps: 262k particles 28.7 / 30.2, 500k 43.6 / 45.9, 700k 57.8 / 54.5, 1M 82.2 /
-// 79.1 (a settled pool 54.0 / 52.3), 2M 149.7 / 140.3, 8.4M 583 / 539. The pressure
-// pass needs 48 registers: at 40 it spills in its loop (1M 91 / 104).
+// Launches whose viscosity pass runs at 48 instead of 40 warps an SM: where that
+// saves a wave, and those of more than three waves (else the last wave costs
+// more than the occupancy gives). Viscosity per substep, us, 40 / 48 warps: 262k
+// particles 28.7 / 30.2, 420k (three waves / two) 38.6 / 36.8, 500k 43.6 / 45.9,
+// 700k 57.8 / 54.5, 1M 82.2 / 79.1 (a settled pool 54.0 / 52.3), 2M 149.7 / 140.3,
+// 8.4M 583 / 539. The pressure pass needs 48 registers: at 40 it spills in its
+// loop (1M 91 / 104).
 constexpr uint32_t kDenseWaves = 3;
 bool dense_form(const LaunchCtx& c, uint32_t ntiles) {
-  return dense_wave(c, ntiles) ||
-         (c.lanes == 1 && c.gather == 2 && ntiles > kDenseWaves * kWaveWarps * c.sms);
+  return c.lanes == 1 && c.gather == 2 &&
+         (ntiles > kDenseWaves * kWaveWarps * c.sms ||
+          (ntiles > kRowsTiles && waves(c, ntiles, kDenseWarps) < waves(c, ntiles, kWaveWarps)));
 }
 
 // List entries a lane of the plain force kernels gathers at once: at least 8,
@@ -2003,9 +2008,8 @@ bool dense_form(const LaunchCtx& c, uint32_t ntiles) {
 constexpr uint32_t kGather8Tiles = 1200;
 constexpr uint32_t kGather3Warps = 32;
 int force_gather(const LaunchCtx& c, uint32_t ntiles) {
-  const auto waves = [&](uint32_t warps) { return (ntiles + warps * c.sms - 1) / (warps * c.sms); };
   const bool three = c.lanes == 1 && ntiles > kDenseWarps * c.sms && ntiles <= kDenseWaves * kWaveWarps * c.sms &&
-                     waves(kGather3Warps) == waves(kWaveWarps);
+                     waves(c, ntiles, kGather3Warps) == waves(c, ntiles, kWaveWarps);
   return std::max(c.gather, ntiles <= kGather8Tiles ? 8 : ntiles <= kRowsTiles ? 4 : three ? 3 : 2);
 }
 

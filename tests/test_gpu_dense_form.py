@@ -11,8 +11,8 @@ from test_gpu_latency_forms import cloud
 
 pytestmark = pytest.mark.gpu
 
-# particles: between 40 and 48 warps an SM; two waves of 32; more than three of 40
-FILLERS = [205000, 250000, 600000]
+# particles: between 40 and 48 warps an SM; two waves of 32; two of 48; more than three of 40
+FILLERS = [205000, 250000, 430000, 600000]
 
 
 @pytest.mark.parametrize("fill", FILLERS)
