@@ -9,7 +9,7 @@
 //                    the state into SoA float4                :484-496
 //   k_cell_table     per cell, its neighbour runs (the bucket walk of
 //                    :331-346 resolved once per cell instead of per particle)
-//   k_density        density / near density and neighbour lists :304-365
+//   k_density_*      density / near density and neighbour lists :304-365
 //   k_pressure       pressure + near pressure over the list   :367-422
 //   k_visc_integrate Jacobi viscosity over the list, integrate, box
 //                    collision, next substep's prediction    :424-464, :81-108
@@ -17,13 +17,18 @@
 // reference's own spatial lookup (HashCell keys, (key, index) order and
 // startIndices, :466-496) from the same predicted positions.
 //
-// The sort key is the internal cell index (sph_device.cuh) modulo the scene
-// size; inside a key bucket particles are ordered by (cell index, particle
-// index), so every cell is a contiguous run of slots and the three cells of
-// an x-row usually one run. Every kernel is a persistent, segmented launch:
-// warps stride over a tile table of (scene, first slot) runs of up to 32
-// particles of one scene, so one launch serves any number of scenes of
-// uneven sizes.
+// The neighbour kernels come in forms for small launches (k_density_rows,
+// k_pressure_coop, k_visc_coop, k_cell_table_rows), the general ones, and ones
+// with another register cap (k_visc_dense); they give the same bits, and the
+// rules beside the launchers choose by the launch's tiles.
+//
+// The sort key is the internal cell index (sph_device.cuh), modulo the scene
+// size where the grid is too large for a table of its own; inside a key bucket
+// particles are ordered by (cell index, particle index), so every cell is a
+// contiguous run of slots and the three cells of an x-row usually one run.
+// Every kernel is a segmented launch: warps stride over a tile table of
+// (scene, first slot) runs of up to 32 particles of one scene, so one launch
+// serves any number of scenes of uneven sizes.
 #include "sph_kernels.h"
 
 #include <algorithm>
@@ -704,9 +709,9 @@ __device__ __forceinline__ void density_store(const SceneDev& S, uint32_t i,
 // density and its list as it goes. Lanes of one cell walk identical runs, so
 // their loads coincide; a lane keeps kWalkBatch candidates in flight (the loads of a
 // run's last batch may pass its end by kPredPad slots, whose pairs are
-// dropped). Issue-bound at large sizes (79% of the slots, 29 warp
-// instructions a candidate of which the hit path takes a third), bound by the
-// latency of its loads below ~300k particles. Against one candidate at a
+// dropped). At large sizes it fills 78% of the issue slots and 70% of the L1 data
+// pipe (26 warp instructions a candidate, of which the hit path takes a third;
+// four wavefronts a 16-byte load), below ~300k particles it waits on its loads. Against one candidate at a
 // time at 32 registers: 131k particles 37 -> 30 us (a step of three substeps
 // 298 -> 248), 500k 93 -> 84, 1M 166 -> 157, 4M 581 -> 567, 8.4M 1149 -> 1161.
 // Batches of 2, 3, 5, 6, 8 and caps of 32, 36, 40 registers (spills) were slower.
