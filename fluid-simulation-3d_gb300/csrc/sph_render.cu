@@ -100,18 +100,21 @@ __device__ __forceinline__ float splat_vy2(const RenderView& v, int py, float y0
   return fm(vy, vy);
 }
 
-// Particles of the scene's slots [first, first + n), one per thread: its
-// colour (by caller index) and its splat into the (depth, index) buffer.
+// Particles of the scene's slots [first, first + n), kSub threads each: its
+// colour (by caller index) and its splat into the (depth, index) buffer, the
+// threads taking its rows in turn (the keys do not depend on the order).
 // A splat of more than kWarpSplat pixels (a particle close to the camera)
 // is drawn by the whole warp, the lanes taking its pixels in turn.
 constexpr int kWarpSplat = 64;
 
+template <int kSub>
 __global__ void k_splat(uint32_t first, uint32_t n, const float4* __restrict__ pos,
                         const float4* __restrict__ vel, RenderView v,
                         unsigned long long* __restrict__ keys,
                         uint32_t* __restrict__ colours) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t lane = threadIdx.x & 31u;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) / kSub;
+  const uint32_t lane = threadIdx.x & 31u, sub = threadIdx.x % kSub;
   bool live = k < n;
   uint32_t id = 0;
   float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -120,7 +123,7 @@ __global__ void k_splat(uint32_t first, uint32_t n, const float4* __restrict__ p
     id = __float_as_uint(p.w);
     live = id < n;
   }
-  if (live) {
+  if (live && sub == 0) {
     const float4 vv = vel[first + k];
     colours[id] = speed_colour(vv.x, vv.y, vv.z);
   }
@@ -158,17 +161,17 @@ __global__ void k_splat(uint32_t first, uint32_t n, const float4* __restrict__ p
   const unsigned long long key =
       (static_cast<unsigned long long>(__float_as_uint(depth)) << 32) | id;
   const float q2 = fm(v.q, v.q);
-  const bool big = live && (xb - xa + 1) * (yb - ya + 1) > kWarpSplat;
+  const bool big = live && (kSub == 32 || (xb - xa + 1) * (yb - ya + 1) > kWarpSplat * kSub);
   if (live && !big) {
     const float idx = fd(1.0f, fs(x1, x0)), idy = fd(1.0f, fs(y1, y0));
-    for (int py = ya; py <= yb; ++py) {
+    for (int py = ya + static_cast<int>(sub); py <= yb; py += kSub) {
       const float vy2 = splat_vy2(v, py, y0, idy);
       unsigned long long* row = keys + static_cast<uint64_t>(py) * v.width;
       for (int px = xa; px <= xb; ++px) splat_pixel(v, px, vy2, x0, idx, q2, key, row);
     }
   }
   // large splats, one at a time across the warp (every lane arrives here)
-  for (uint32_t m = __ballot_sync(0xffffffffu, big); m; m &= m - 1u) {
+  for (uint32_t m = __ballot_sync(0xffffffffu, big && sub == 0); m; m &= m - 1u) {
     const int src = __ffs(m) - 1;
     const int bxa = __shfl_sync(0xffffffffu, xa, src), bxb = __shfl_sync(0xffffffffu, xb, src);
     const int bya = __shfl_sync(0xffffffffu, ya, src), byb = __shfl_sync(0xffffffffu, yb, src);
@@ -191,12 +194,15 @@ __global__ void k_splat(uint32_t first, uint32_t n, const float4* __restrict__ p
 // clear colour and depth 1, as 16-byte words; a covered key is put back to
 // empty for the next frame (no clear of the whole buffer). The outputs may be
 // pinned host memory: the words then go over the link from here, which bounds
-// the frame (1080p, 16.6 MB, 131,072 particles: 117 us; 136 us when the keys
-// were cleared, the image resolved on the device and copied).
+// the frame (1080p, 16.6 MB: 88 us here). It starts beside k_splat and waits for
+// it: 2 us a frame. (131,072 particles at 1080p: 136 us when the keys were
+// cleared, the image resolved on the device and copied, 120 straight into pinned
+// images, 115 with this and the split splats.)
 __global__ void k_resolve(uint32_t pixels, unsigned long long* __restrict__ keys,
                           const uint32_t* __restrict__ colours, uint32_t clear,
                           uint32_t* __restrict__ rgba, float* __restrict__ depth) {
   const uint32_t i = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // for k_splat, beside which it starts
   if (i >= pixels) return;
   const uint32_t m = min(4u, pixels - i);
   uint32_t c[4];
@@ -224,6 +230,20 @@ __global__ void k_resolve(uint32_t pixels, unsigned long long* __restrict__ keys
   }
 }
 
+// Threads a splat takes: the fewer particles an image of some size holds, the
+// more pixels each covers and the fewer threads there would be, one a particle,
+// walking its pixels one after another. By pixels of the image per particle;
+// frames into pinned memory, us, by 1 / 2 / 4 / 8 / 32 threads:
+//   1920x1080: 4k 153 / 127 / 114 / 109 / 105, 16k 126 / 114 / 108 / 108 / 108 (a pool
+//   167 / 140 / 126 / 118 / 113), 65k 124 / 113 / 113 / 112 / 125 (pool 150 / 133 / 126 /
+//   119 / 132), 131k 118 / 117 / 115 / 115 / 147, 262k 118 / 117 / 117 / 126 / 189 (pool
+//   148 / 134 / 125 / 132 / 198), 524k 125 / 124 / 127 / 151, 1M 124 / 128 / 146 / 190;
+//   640x360: 131k 25.5 / 26.7 / 29.1 / 34.5
+// (the link's share of a 1920x1080 frame is 85).
+int splat_threads(uint64_t pixels, uint64_t n) {
+  return pixels >= 200 * n ? 32 : pixels >= 20 * n ? 8 : pixels >= 10 * n ? 4 : pixels >= 3 * n ? 2 : 1;
+}
+
 }  // namespace
 
 cudaError_t launch_render(uint32_t first, uint32_t n, const float4* pos, const float4* vel,
@@ -232,12 +252,27 @@ cudaError_t launch_render(uint32_t first, uint32_t n, const float4* pos, const f
                           cudaStream_t st) {
   cudaError_t e = cudaSuccess;
   if (n) {
-    k_splat<<<(n + 255) / 256, 256, 0, st>>>(first, n, pos, vel, view, keys, colours);
+    const int sub = splat_threads(static_cast<uint64_t>(view.width) * view.height, n);
+    auto kern = sub == 32  ? k_splat<32>
+                : sub == 8 ? k_splat<8>
+                : sub == 4 ? k_splat<4>
+                : sub == 2 ? k_splat<2>
+                           : k_splat<1>;
+    const uint32_t per = 256u / static_cast<uint32_t>(sub);
+    kern<<<(n + per - 1) / per, 256, 0, st>>>(first, n, pos, vel, view, keys, colours);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   const uint32_t px = view.width * view.height;
-  k_resolve<<<(px + 1023) / 1024, 256, 0, st>>>(px, keys, colours, view.clear, rgba, depth);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((px + 1023) / 1024);
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = n ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k_resolve, px, keys, colours, view.clear, rgba, depth);
 }
 
 }  // namespace sph
