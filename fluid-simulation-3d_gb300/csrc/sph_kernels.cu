@@ -2012,8 +2012,11 @@ bool dense_form(const LaunchCtx& c, uint32_t ntiles) {
 // 237, 317 / 314; but 332k 405 / 410, 380k 441 / 462, 500k 565 / 565.
 constexpr uint32_t kGather8Tiles = 1200;
 constexpr uint32_t kGather3Warps = 32;
+constexpr int kGatherBlock = 512;  // the largest block 127 registers a thread leave
 int force_gather(const LaunchCtx& c, uint32_t ntiles) {
-  const bool three = c.lanes == 1 && ntiles > kDenseWarps * c.sms && ntiles <= kDenseWaves * kWaveWarps * c.sms &&
+  if (c.block_force > kGatherBlock) return c.gather;
+  const bool three = c.lanes == 1 && ntiles > kDenseWarps * c.sms &&
+                     ntiles <= kDenseWaves * kWaveWarps * c.sms &&
                      waves(c, ntiles, kGather3Warps) == waves(c, ntiles, kWaveWarps);
   return std::max(c.gather, ntiles <= kGather8Tiles ? 8 : ntiles <= kRowsTiles ? 4 : three ? 3 : 2);
 }

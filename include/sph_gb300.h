@@ -76,7 +76,8 @@ typedef struct sph_tuning {
                          its list; agrees with 32 to rounding)            */
   int32_t gather;     /* neighbour-list entries whose gathers the force
                          kernels issue together: 2, 3, 4 or 8 (default 2;
-                         small launches issue 4 or 8 at least). Results do
+                         small launches issue 4 or 8 at least, some of a
+                         few waves 3, in blocks of up to 512). Results do
                          not depend on it                                 */
   int32_t force_block; /* threads per block of the pressure and viscosity
                           kernels (multiple of 32, 32..1024); 0 = block   */
