@@ -167,4 +167,32 @@ __device__ __forceinline__ uint32_t table_key(const SceneDev& S, uint32_t cell) 
 // are not written and must not be read).
 constexpr uint32_t kRunMerged = 0x80000000u;
 
+// Programmatic dependent launch: the substep kernels are launched with
+// programmatic stream serialisation (launch_pdl), so each one is scheduled
+// while its predecessor's last wave runs. Every such kernel first lets its
+// own successor be scheduled (pdl_launch), may then read what no kernel of a
+// step writes -- the tile table and the scene constants, uploaded before the
+// step began -- and waits for its predecessor to complete with its memory
+// visible (pdl_wait: a hardware dependency, not a spin) before it touches
+// anything else. Reading the tables before the wait takes two dependent loads
+// off the chain of each of the seven to eight kernels of a substep. Without the launch
+// attribute both are no-ops; a second wait returns at once.
+//
+// The wait hands its argument through: the index or the address that the
+// kernel's loads are formed from. What the predecessor writes reaches a kernel
+// through `const __restrict__` pointers and loads the compiler takes for pure
+// functions of their address, which a memory clobber alone does not hold back;
+// an address that hangs on the wait's result does.
+__device__ __forceinline__ void pdl_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t pdl_wait(uint32_t x) {
+  asm volatile("griddepcontrol.wait;" : "+r"(x) :: "memory");
+  return x;
+}
+__device__ __forceinline__ uint32_t pdl_enter(uint32_t x) {
+  pdl_launch();
+  return pdl_wait(x);
+}
+
 }  // namespace sph

@@ -72,27 +72,6 @@ __device__ __forceinline__ void flag(uint32_t* status, uint32_t f) {
   atomicOr(status, f);
 }
 
-// Programmatic dependent launch: the substep kernels are launched with
-// programmatic stream serialisation (launch_pdl), so each one is scheduled
-// while its predecessor's last wave runs. Every such kernel first lets its
-// own successor be scheduled (pdl_launch), may then read what no kernel of a
-// step writes -- the tile table and the scene constants, uploaded before the
-// step began -- and waits for its predecessor to complete with its memory
-// visible (pdl_wait: a hardware dependency, not a spin) before it touches
-// anything else. Reading the tables before the wait takes two dependent loads
-// off the chain of each of the seven to eight kernels of a substep. Without the launch
-// attribute both are no-ops; a second wait returns at once.
-__device__ __forceinline__ void pdl_launch() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void pdl_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-__device__ __forceinline__ void pdl_enter() {
-  pdl_launch();
-  pdl_wait();
-}
-
 // Entry k of slot i's neighbour list. Groups of 32 slots own kNbrCap rows of
 // 32 entries (8 KB), so a warp's appends and loads of one entry are contiguous
 // and all its rows lie side by side. A row per entry number over all slots
@@ -127,10 +106,11 @@ __device__ __forceinline__ void store_state(float4* __restrict__ rec, float2* __
 }
 __device__ __forceinline__ void load_rec(const float4* __restrict__ rec,
                                          uint32_t j, float4& a, float4& b) {
-  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y),
-        "=f"(b.z), "=f"(b.w)
-      : "l"(rec + 2ull * j));
+  asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y),
+                 "=f"(b.z), "=f"(b.w)
+               : "l"(rec + 2ull * j)
+               : "memory");
 }
 __device__ __forceinline__ void store_rec(float4* __restrict__ rec, uint32_t i,
                                           float4 a, float4 b) {
@@ -271,10 +251,9 @@ __global__ void k_scenes(const __grid_constant__ SceneChunk<N> chunk, uint32_t w
 // its first tile with the next). 16 B a tile, so bound by the launch.
 __global__ void k_tiles(const SceneDev* __restrict__ scene_table, uint32_t scenes, uint32_t ntiles,
                         uint2* __restrict__ tiles_old, uint2* __restrict__ tiles_new) {
-  pdl_wait();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ntiles) return;
-  uint32_t lo = 0, hi = scenes;  // tile0 of lo is <= t, of hi (if any) > t
+  uint32_t lo = 0, hi = pdl_wait(scenes);  // tile0 of lo is <= t, of hi (if any) > t
   while (hi - lo > 1u) {
     const uint32_t mid = lo + (hi - lo) / 2u;
     if (scene_table[mid].tile0 <= t) lo = mid; else hi = mid;
@@ -306,8 +285,7 @@ __global__ void k_predict_hash(const uint2* __restrict__ tiles, uint32_t ntiles,
   for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const SceneDev S = scenes[tile_scene(tile)];  // registers, not reloads
-    pdl_wait();
-    const uint32_t s = tile.y + lane;
+    const uint32_t s = pdl_wait(tile.y) + lane;
     const bool live = lane < tile_len(tile);
     uint32_t key = 0, cell = 0, id = 0;
     if (live) {
@@ -364,8 +342,7 @@ __global__ void __launch_bounds__(kScanThreads)
 k_scan_reduce(const uint32_t* __restrict__ count, uint32_t len,
               uint32_t* __restrict__ partial) {
   static_assert(kScanItems == 4, "one uint4 of counts per thread");
-  pdl_enter();
-  const uint32_t b0 = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
+  const uint32_t b0 = pdl_enter(blockIdx.x * kScanBlock + threadIdx.x * kScanItems);
   const uint4 v = load_counts(count, b0, len);
   uint32_t total;
   block_excl_scan(v.x + v.y + v.z + v.w, &total);
@@ -375,10 +352,10 @@ k_scan_reduce(const uint32_t* __restrict__ count, uint32_t len,
 __global__ void __launch_bounds__(kScanThreads)
 k_scan_partials(uint32_t* __restrict__ partial, uint32_t nb,
                 uint32_t* __restrict__ start, uint32_t len) {
-  pdl_enter();
+  const uint32_t thread = pdl_enter(threadIdx.x);
   uint32_t carry = 0;
   for (uint32_t c = 0; c < nb; c += kScanThreads) {
-    const uint32_t i = c + threadIdx.x;
+    const uint32_t i = c + thread;
     const uint32_t v = i < nb ? partial[i] : 0u;
     uint32_t total;
     const uint32_t ex = block_excl_scan(v, &total);
@@ -399,12 +376,12 @@ k_scan_down(uint32_t* __restrict__ count, uint32_t len,
             const uint32_t* __restrict__ partial, uint32_t nb, int fold,
             uint32_t* __restrict__ start) {
   __shared__ uint32_t warp_scan[kScanThreads / 32], warp_fold[kScanThreads / 32];
-  pdl_enter();
-  const uint32_t b0 = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
+  const uint32_t block = pdl_enter(blockIdx.x);
+  const uint32_t b0 = block * kScanBlock + threadIdx.x * kScanItems;
   const uint4 v = load_counts(count, b0, len);
   uint32_t f = 0;
   if (fold) {
-    for (uint32_t c = threadIdx.x; c < blockIdx.x; c += kScanThreads) f += partial[c];
+    for (uint32_t c = threadIdx.x; c < block; c += kScanThreads) f += partial[c];
   }
   const uint32_t s = v.x + v.y + v.z + v.w;
   const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
@@ -423,7 +400,7 @@ k_scan_down(uint32_t* __restrict__ count, uint32_t len,
     block_total += ws;
     base += warp_fold[u];
   }
-  if (!fold) base = partial[blockIdx.x];
+  if (!fold) base = partial[block];
   uint32_t run = base + before + incl - s;
   if (b0 + 4u <= len) {
     uint4 o;
@@ -444,7 +421,7 @@ k_scan_down(uint32_t* __restrict__ count, uint32_t len,
       run += vv[k];
     }
   }
-  if (fold && blockIdx.x + 1 == nb && threadIdx.x == 0) start[len] = base + block_total;
+  if (fold && block + 1 == nb && threadIdx.x == 0) start[len] = base + block_total;
 }
 
 // ----------------------------------------------------------------- scatter
@@ -457,8 +434,7 @@ __global__ void k_scatter(const uint2* __restrict__ tiles, uint32_t ntiles,
   const uint32_t lane = lane_id();
   for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
-    pdl_wait();
-    const uint32_t s = tile.y + lane;
+    const uint32_t s = pdl_wait(tile.y) + lane;
     if (lane >= tile_len(tile)) continue;
     const uint4 kr = keyrank[s];
     const uint32_t dst = start[kr.x] + kr.y;
@@ -495,8 +471,7 @@ __global__ void k_reorder(const uint2* __restrict__ tiles, uint32_t ntiles,
   for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const SceneDev S = scenes[tile_scene(tile)];  // registers, not reloads
-    pdl_wait();
-    const uint32_t slot = tile.y + lane;
+    const uint32_t slot = pdl_wait(tile.y) + lane;
     if (lane >= tile_len(tile)) continue;
     const uint2 me = tmp_hi[slot];
     const uint32_t src = tmp_src[slot];
@@ -631,9 +606,9 @@ k_cell_table(const uint2* __restrict__ tiles, uint32_t ntiles,
   for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const SceneDev S = scenes[tile_scene(tile)];  // registers, not reloads
-    pdl_wait();
+    const uint32_t first = pdl_wait(tile.y);
     if (S.direct) continue;  // its rows come from the start table
-    const uint32_t i = tile.y + lane;
+    const uint32_t i = first + lane;
     const bool live = lane < tile_len(tile);
     const bool leader = live && cell_first[i] == i;
     const uint32_t lmask = __ballot_sync(kFull, leader);
@@ -643,7 +618,7 @@ k_cell_table(const uint2* __restrict__ tiles, uint32_t ntiles,
     const uint32_t kmax = fastmod(0xffffffffu, S.fm, S.n);  // key of 2^32 - 1
     for (uint32_t q = lane; q < pairs; q += 32) {
       const uint32_t c = q / 9u, w = q - c * 9u;
-      cell_row(S, tile.y + lead[c], w, kmax, hash_s, start, cell_tab);
+      cell_row(S, first + lead[c], w, kmax, hash_s, start, cell_tab);
     }
     __syncwarp();  // the next tile rewrites the leader list
   }
@@ -662,9 +637,8 @@ k_cell_table_rows(const uint2* __restrict__ tiles, uint32_t ntiles,
   for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const uint2 tile = tiles[t];
     const SceneDev S = scenes[tile_scene(tile)];
-    pdl_wait();
+    const uint32_t i = pdl_wait(tile.y) + lane;
     if (S.direct) continue;  // its rows come from the start table
-    const uint32_t i = tile.y + lane;
     if (lane < tile_len(tile) && cell_first[i] == i)
       cell_row(S, i, w, fastmod(0xffffffffu, S.fm, S.n), hash_s, start, cell_tab);
   }
@@ -735,9 +709,8 @@ k_density_walk(const uint2* __restrict__ tiles, uint32_t ntiles,
                       : kTables == kTablesBuckets ? false
                                                   : S.direct != 0u;
     const float cut = S.cut_le, r = S.r;
-    pdl_wait();
+    const uint32_t i = pdl_wait(tile.y) + lane;
     if (lane >= tile_len(tile)) continue;
-    const uint32_t i = tile.y + lane;
     const float4 me = pred[i];
     const float2 npxy = make_float2(-me.x, -me.y);
     float s2 = S.r2, s3 = S.r2 * r;  // self: w = r
@@ -847,9 +820,8 @@ k_density_rows(const uint2* __restrict__ tiles, uint32_t ntiles,
     const bool direct = kTables == kTablesDirect    ? true
                       : kTables == kTablesBuckets ? false
                                                   : S.direct != 0u;
-    pdl_wait();
     const bool live = lane < tile_len(tile);
-    const uint32_t i = tile.y + (live ? lane : 0u);
+    const uint32_t i = pdl_wait(tile.y) + (live ? lane : 0u);
     const float4 me = pred[i];
     const uint32_t cell = __float_as_uint(me.w);
     const uint32_t cf = kTables == kTablesDirect ? 0u : cell_first[i];
@@ -961,10 +933,10 @@ __global__ void k_density(const uint2* __restrict__ tiles, uint32_t ntiles,
                           float4* __restrict__ dens_b,
                           uint32_t* __restrict__ nbr,
                           uint32_t* __restrict__ ncount) {
-  pdl_enter();
+  const uint32_t warp = pdl_enter(warp_id_global());
   const uint32_t lane = lane_id();
   const uint32_t lt_mask = (1u << lane) - 1u;
-  for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
+  for (uint32_t t = warp; t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const SceneDev S = scenes[tile_scene(tile)];  // registers, not reloads
     const uint32_t i = tile.y + lane;
@@ -1129,13 +1101,13 @@ __global__ void k_pressure(const uint2* __restrict__ tiles, uint32_t ntiles,
   for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const SceneDev S = scenes[tile_scene(tile)];  // registers, not reloads
-    pdl_wait();
+    const uint32_t first = pdl_wait(tile.y);
 #pragma unroll 1
     for (uint32_t h = 0; h < kLanes; ++h) {
       const uint32_t li = h * kPer + lane % kPer;
       if (kLanes == 1 && li >= tile_len(tile)) break;
       const bool live = li < tile_len(tile);
-      const uint32_t i = tile.y + (live ? li : 0u);
+      const uint32_t i = first + (live ? li : 0u);
       const float4 pi = pred[i];
       const float3 p = make_float3(pi.x, pi.y, pi.z);
       const float2 di = dens_a[i];
@@ -1229,9 +1201,8 @@ k_pressure_coop(const uint2* __restrict__ tiles, uint32_t ntiles,
     const uint32_t sub = v % kCoopSub * kCoopPer, len = tile_len(tile);
     if (sub >= len) continue;
     const SceneDev S = scenes[tile_scene(tile)];
-    pdl_wait();
     const bool live = sub + pp < len;
-    const uint32_t i = tile.y + min(sub + pp, len - 1u);
+    const uint32_t i = pdl_wait(tile.y) + min(sub + pp, len - 1u);
     const float4 pi = pred[i];
     const float3 p = make_float3(pi.x, pi.y, pi.z);
     const float2 di = dens_a[i];
@@ -1356,11 +1327,12 @@ __device__ __forceinline__ void visc_tiles(
     uint4* __restrict__ keyrank, float4* __restrict__ dbg_velv,
     uint32_t* status) {
   static_assert(kLanes == 1 || kLanes == 2, "one or two lanes per particle");
-  pdl_enter();  // (the early table read costs this kernel registers: 8.4M 599 -> 627 us)
+  // (the early table read costs this kernel registers: 8.4M 599 -> 627 us)
+  const uint32_t warp = pdl_enter(warp_id_global());
   const uint32_t lane = lane_id();
   constexpr uint32_t kPer = 32 / kLanes;  // particles per pass
   const uint32_t sub = lane / kPer;       // this lane's share of the list
-  for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
+  for (uint32_t t = warp; t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const SceneDev S = scenes[tile_scene(tile)];  // registers, not reloads
 #pragma unroll 1
@@ -1476,9 +1448,8 @@ __global__ void __launch_bounds__(kCoopBlock) k_visc_coop(
     const uint32_t sub = v % kCoopSub * kCoopPer, len = tile_len(tile);
     if (sub >= len) continue;
     const SceneDev S = scenes[tile_scene(tile)];
-    pdl_wait();
     const bool in_tile = sub + pp < len;
-    const uint32_t i = tile.y + min(sub + pp, len - 1u);
+    const uint32_t i = pdl_wait(tile.y) + min(sub + pp, len - 1u);
     float4 pi, vi;
     load_rec(rec_v, i, pi, vi);
     const float3 p = make_float3(pi.x, pi.y, pi.z);
@@ -1608,8 +1579,7 @@ __global__ void __launch_bounds__(256) k_export_rows(uint32_t first, uint32_t n,
                                                      float* __restrict__ odens) {
   __shared__ __align__(16) float buf[8][96];
   const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  const uint32_t i0 = (blockIdx.x * 8u + w) * 32u;
-  pdl_wait();
+  const uint32_t i0 = pdl_wait((blockIdx.x * 8u + w) * 32u);
   if (i0 >= n) return;
   const uint32_t rows = min(32u, n - i0);
   const uint32_t s = lane < rows ? slot_of[i0 + lane] : first;
@@ -1645,9 +1615,9 @@ __global__ void k_ref_hash(const uint2* __restrict__ tiles, uint32_t ntiles,
                            uint2* __restrict__ keyrank,
                            uint32_t* __restrict__ ohash,
                            uint32_t* __restrict__ okey, uint32_t* status) {
-  pdl_enter();
+  const uint32_t warp = pdl_enter(warp_id_global());
   const uint32_t lane = lane_id();
-  for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
+  for (uint32_t t = warp; t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const SceneDev S = scenes[tile_scene(tile)];
     const uint32_t s = tile.y + lane;
@@ -1678,9 +1648,9 @@ __global__ void k_ref_scatter(const uint2* __restrict__ tiles, uint32_t ntiles,
                               const uint32_t* __restrict__ start,
                               uint32_t total, uint32_t* __restrict__ tmp,
                               uint32_t* status) {
-  pdl_enter();
+  const uint32_t warp = pdl_enter(warp_id_global());
   const uint32_t lane = lane_id();
-  for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
+  for (uint32_t t = warp; t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const uint32_t s = tile.y + lane;
     if (lane >= tile_len(tile)) continue;
@@ -1698,9 +1668,9 @@ __global__ void k_ref_order(const uint2* __restrict__ tiles, uint32_t ntiles,
                             const uint32_t* __restrict__ start,
                             const uint32_t* __restrict__ tmp,
                             uint32_t* __restrict__ sorted) {
-  pdl_enter();
+  const uint32_t warp = pdl_enter(warp_id_global());
   const uint32_t lane = lane_id();
-  for (uint32_t t = warp_id_global(); t < ntiles; t += warps_total()) {
+  for (uint32_t t = warp; t < ntiles; t += warps_total()) {
     const uint2 tile = tiles[t];
     const uint32_t s = tile.y + lane;
     if (lane >= tile_len(tile)) continue;
@@ -1847,7 +1817,7 @@ k_import_rows(uint32_t first, uint32_t n, const float* __restrict__ ipos,
     const SceneDev S = *scene;
     uint32_t key = 0, cell = 0;
     if (live) predict_key(S, p4, v4, key, cell);
-    pdl_wait();  // for k_clear
+    key = pdl_wait(key);  // for k_clear
     const uint32_t r = aggregated_rank(count, key, live);
     if (live) keyrank[first + k] = make_uint4(key, r, cell, k);
   }
@@ -1858,7 +1828,7 @@ k_import_rows(uint32_t first, uint32_t n, const float* __restrict__ ipos,
 // ------------------------------------------------------------- launchers
 // Substep kernels go out with programmatic stream serialisation: the next
 // kernel is scheduled during its predecessor's last wave and waits for it in
-// pdl_enter(), which hides the launch and ramp-up between the seven to nine
+// pdl_wait(), which hides the launch and ramp-up between the seven to nine
 // kernels of a substep (inside a graph these become programmatic edges).
 template <class... KArgs, class... Args>
 cudaError_t launch_pdl_smem(bool pdl, void (*kernel)(KArgs...), uint32_t grid, int block,

@@ -30,6 +30,7 @@
 
 #include <cstdint>
 
+#include "sph_device.cuh"
 #include "sph_render.h"
 
 namespace sph {
@@ -112,7 +113,7 @@ __global__ void k_splat(uint32_t first, uint32_t n, const float4* __restrict__ p
                         const float4* __restrict__ vel, RenderView v,
                         unsigned long long* __restrict__ keys,
                         uint32_t* __restrict__ colours) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_launch();
   const uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) / kSub;
   const uint32_t lane = threadIdx.x & 31u, sub = threadIdx.x % kSub;
   bool live = k < n;
@@ -201,8 +202,8 @@ __global__ void k_splat(uint32_t first, uint32_t n, const float4* __restrict__ p
 __global__ void k_resolve(uint32_t pixels, unsigned long long* __restrict__ keys,
                           const uint32_t* __restrict__ colours, uint32_t clear,
                           uint32_t* __restrict__ rgba, float* __restrict__ depth) {
-  const uint32_t i = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // for k_splat, beside which it starts
+  // waits for k_splat, beside which it starts
+  const uint32_t i = pdl_wait(4u * (blockIdx.x * blockDim.x + threadIdx.x));
   if (i >= pixels) return;
   const uint32_t m = min(4u, pixels - i);
   uint32_t c[4];
