@@ -790,11 +790,12 @@ int Engine::Render(uint32_t id, const sph_view& v, uint8_t* rgba, float* depth,
   if (!render_empty_)
     SPH_CUDA(cudaMemsetAsync(d_rkeys_, 0xff, sizeof(unsigned long long) * render_pixels_, st),
              "clear image keys");
-  render_empty_ = false;  // until this frame's resolve is queued
+  // until this frame's resolve has run (one queued into a caller's capture,
+  // which the wait below refuses, never does)
+  render_empty_ = false;
   SPH_CUDA(launch_render(old_base_[id], scenes_[id].n, d_pos_[cur_], d_vel_[cur_], rv,
                          d_rkeys_, d_rcolour_, direct ? hc : d_rrgba_, direct ? hz : d_rdepth_, st),
            "render kernels");
-  render_empty_ = true;
   if (rgba && !direct)
     SPH_CUDA(cudaMemcpyAsync(rgba, d_rrgba_, 4 * pixels, cudaMemcpyDeviceToHost, st),
              "download image");
@@ -802,6 +803,7 @@ int Engine::Render(uint32_t id, const sph_view& v, uint8_t* rgba, float* depth,
     SPH_CUDA(cudaMemcpyAsync(depth, d_rdepth_, 4 * pixels, cudaMemcpyDeviceToHost, st),
              "download depth");
   SPH_CUDA(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+  render_empty_ = true;
   return SPH_OK;
 }
 
