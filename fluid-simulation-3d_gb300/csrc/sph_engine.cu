@@ -27,6 +27,16 @@ template <class T> T* DeviceAlias(T* p) {
   return static_cast<T*>(a.devicePointer);
 }
 
+// Whether a caller is capturing `st`. (The question itself fails for the legacy
+// stream while another stream is being captured; the launches made then report
+// that to the caller.)
+bool Capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return false;
+}
+
 const float* Aligned16(const float* p) {
   return (reinterpret_cast<std::uintptr_t>(p) & 15u) ? nullptr : p;
 }
@@ -392,7 +402,10 @@ int Engine::Load(uint32_t id, const float* pos3, const float* vel3,
                                 predict ? count_extent_ : 0u, ctx_.keyrank, st),
              "import kernel");
     if (predict) {
-      carry_valid_ = true;
+      // Captured by the caller, the kernel has not run when the next step is
+      // called: that step predicts for whatever state it finds. (The graph
+      // predicts all the same, for steps that follow a later launch of it.)
+      carry_valid_ = !Capturing(st);
       count_extent_ = table_total_;
     }
   } else if (!device_ptrs && pos3) {
