@@ -1982,7 +1982,7 @@ bool dense_form(const LaunchCtx& c, uint32_t ntiles) {
 // 237, 317 / 314; but 332k 405 / 410, 380k 441 / 462, 500k 565 / 565.
 constexpr uint32_t kGather8Tiles = 1200;
 constexpr uint32_t kGather3Warps = 32;
-constexpr int kGatherBlock = 512;  // the largest block 127 registers a thread leave
+constexpr int kGatherBlock = 512;  // larger ones gather what the tuning asks for, if it fits
 int force_gather(const LaunchCtx& c, uint32_t ntiles) {
   if (c.block_force > kGatherBlock) return c.gather;
   const bool three = c.lanes == 1 && ntiles > kDenseWarps * c.sms &&
@@ -2081,6 +2081,21 @@ auto visc_kernel(int gather, int lanes) {
   return lanes == 2 ? visc_kernel<kTables, 2>(gather) : visc_kernel<kTables, 1>(gather);
 }
 
+// pick(gather), or the kernel of the next smaller batch that a block of `block`
+// threads has the registers for: 4 entries take up to 78 a thread, 8 up to 127,
+// where 1,024 threads leave 64 (two take 63 at most). 256 threads fit whatever
+// a kernel takes and need no question. The results do not depend on the batch.
+template <class Pick> auto fitting_kernel(Pick pick, int gather, int block) {
+  for (;;) {
+    const auto kern = pick(gather);
+    cudaFuncAttributes a{};
+    if (gather == 2 || block <= 256 ||
+        (cudaFuncGetAttributes(&a, kern) == cudaSuccess && a.maxThreadsPerBlock >= block))
+      return kern;
+    gather = gather == 8 ? 4 : gather - 1;
+  }
+}
+
 cudaError_t launch_pressure(const LaunchCtx& c, const Tiles& tiles,
                             cudaStream_t st) {
   if (tiles.n == 0) return cudaSuccess;
@@ -2093,10 +2108,12 @@ cudaError_t launch_pressure(const LaunchCtx& c, const Tiles& tiles,
                       tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab,
                       c.dens_a, c.dens_b, c.nbr, c.ncount, c.vel2, c.rec_v, c.dbg_accp,
                       c.dbg_velp);
-  const int b = c.block_force, gather = force_gather(c, tiles.n);
-  auto kern = c.tables == kTablesDirect    ? pressure_kernel<kTablesDirect>(gather, c.lanes)
-              : c.tables == kTablesBuckets ? pressure_kernel<kTablesBuckets>(gather, c.lanes)
-                                           : pressure_kernel<kTablesMixed>(gather, c.lanes);
+  const int b = c.block_force;
+  auto kern = fitting_kernel([&](int gather) {
+    return c.tables == kTablesDirect    ? pressure_kernel<kTablesDirect>(gather, c.lanes)
+           : c.tables == kTablesBuckets ? pressure_kernel<kTablesBuckets>(gather, c.lanes)
+                                        : pressure_kernel<kTablesMixed>(gather, c.lanes);
+  }, force_gather(c, tiles.n), b);
   // Started early beside k_density_rows' blocks this kernel would run with the
   // L1 their shared memory leaves it (37k particles: 9 us a substep).
   return launch_pdl(c.pdl && !rows_form(c, tiles.n) && !one_wave(c, tiles.n), kern,
@@ -2118,13 +2135,16 @@ cudaError_t launch_visc_integrate(const LaunchCtx& c, const Tiles& tiles,
                       tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab, c.nbr,
                       c.ncount, c.rec_v, c.pos2, c.vel2, write_out ? c.out4 : nullptr, fuse_next,
                       c.count, c.keyrank, c.dbg_velv, c.status);
-  const int b = c.block_force, gather = force_gather(c, tiles.n);
-  auto kern = dense_form(c, tiles.n) ? (c.tables == kTablesDirect    ? k_visc_dense<kTablesDirect>
-                                        : c.tables == kTablesBuckets ? k_visc_dense<kTablesBuckets>
-                                                                     : k_visc_dense<kTablesMixed>)
-              : c.tables == kTablesDirect  ? visc_kernel<kTablesDirect>(gather, c.lanes)
-              : c.tables == kTablesBuckets ? visc_kernel<kTablesBuckets>(gather, c.lanes)
-                                           : visc_kernel<kTablesMixed>(gather, c.lanes);
+  const int b = c.block_force;
+  auto kern = dense_form(c, tiles.n)
+                  ? (c.tables == kTablesDirect    ? k_visc_dense<kTablesDirect>
+                     : c.tables == kTablesBuckets ? k_visc_dense<kTablesBuckets>
+                                                  : k_visc_dense<kTablesMixed>)
+                  : fitting_kernel([&](int gather) {
+    return c.tables == kTablesDirect    ? visc_kernel<kTablesDirect>(gather, c.lanes)
+           : c.tables == kTablesBuckets ? visc_kernel<kTablesBuckets>(gather, c.lanes)
+                                        : visc_kernel<kTablesMixed>(gather, c.lanes);
+  }, force_gather(c, tiles.n), b);
   return launch_pdl(c.pdl && !one_wave(c, tiles.n), kern, grid_for(tiles.n, b, c.max_blocks), b,
                     st, tiles.d, tiles.n, c.scenes, c.pred, c.start, c.cell_first, c.cell_tab, c.nbr,
                     c.ncount, c.rec_v, c.rec_b, c.pos2, c.vel2,
