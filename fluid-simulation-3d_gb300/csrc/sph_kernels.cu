@@ -1228,8 +1228,10 @@ k_pressure_coop(const uint2* __restrict__ tiles, uint32_t ntiles,
             const float dx = q[u].x - p.x, dy = q[u].y - p.y, dz = q[u].z - p.z;
             const float d2 = dist2(dx, dy, dz);
             const float tsum = pressure_term(S, d2, Pi, Pni, b[u]);
+            // (a coincident pair's term is tsum, along y: -0 * 1 leaves x and z
+            // what they are also where tsum is infinite)
             row[k0 + 4u * u] = d2 > 0.0f ? make_float4(dx, dy, dz, tsum * rsqrtf(d2))
-                                         : make_float4(0.0f, 1.0f, 0.0f, tsum);
+                                         : make_float4(-0.0f, tsum, -0.0f, 1.0f);
           }
         }
       }
@@ -1472,7 +1474,7 @@ __global__ void __launch_bounds__(kCoopBlock) k_visc_coop(
             row[k0 + 4u * u] = d2 <= S.cut_lt
                                    ? make_float4(vj[u].x - vi.x, vj[u].y - vi.y, vj[u].z - vi.z,
                                                  w * w * w)
-                                   : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                                   : make_float4(-0.0f, -0.0f, -0.0f, 1.0f);  // no change
           }
         }
       }
