@@ -228,6 +228,57 @@ __device__ __forceinline__ void walk_runs(const SceneDev& S,
   }
 }
 
+// One row of the same walk for the latency forms, visit(j, q, true) for its
+// particles in the same order, kBatch candidates in flight (one at a time, a
+// candidate costs an L2 round trip; the last batch repeats the run's last
+// particle with false). k: the table entry of the row's middle cell in a
+// direct table; tab: the row's entries in the cell table. A run is walked if
+// enter(its length) says so.
+template <int kTables, uint32_t kBatch, class Enter, class F>
+__device__ __forceinline__ void walk_row(bool direct, const uint32_t* __restrict__ start,
+                                         uint32_t k, const uint2* __restrict__ tab,
+                                         const float4* __restrict__ pred, Enter&& enter,
+                                         F&& visit) {
+  auto run = [&](uint32_t j, uint32_t e) {
+    if (!enter(e - j)) return;
+    for (; j < e; j += kBatch) {
+      float4 q[kBatch];
+#pragma unroll
+      for (uint32_t u = 0; u < kBatch; ++u) q[u] = __ldg(pred + min(j + u, e - 1u));
+#pragma unroll
+      for (uint32_t u = 0; u < kBatch; ++u) visit(j + u, q[u], j + u < e);
+    }
+  };
+  if (kTables == kTablesDirect || (kTables == kTablesMixed && direct)) {
+    run(__ldg(start + k - 1), __ldg(start + k + 2));
+    return;
+  }
+  const uint2 m = __ldg(tab);
+  if (m.y & kRunMerged) {
+    run(m.x, m.x + (m.y & ~kRunMerged));
+    return;
+  }
+#pragma unroll 1
+  for (int c = 0; c < 3; ++c) {
+    const uint2 x = c ? __ldg(tab + c) : m;
+    run(x.x, x.x + x.y);
+  }
+}
+
+// walk_runs by walk_row.
+template <int kTables, uint32_t kBatch, class F>
+__device__ __forceinline__ void walk_rows(const SceneDev& S, const uint32_t* __restrict__ start,
+                                          const uint2* __restrict__ cell_tab, uint32_t cf,
+                                          uint32_t cell, const float4* __restrict__ pred,
+                                          F&& visit) {
+#pragma unroll 1
+  for (uint32_t w = 0; w < 9u; ++w)
+    walk_row<kTables, kBatch>(S.direct != 0u, start,
+                              S.tbase + cell + (w / 3u - 1u) * S.gwy + (w % 3u - 1u) * S.gwz,
+                              cell_tab + static_cast<uint64_t>(cf) * 27u + 3u * w, pred,
+                              [](uint32_t) { return true; }, visit);
+}
+
 // --------------------------------------------------------- scenes and tiles
 // Part of the scene table as a kernel parameter (up to the parameters' 4 KB,
 // and 32 KB for large batches): it needs no staging memory and no wait, and is
@@ -793,11 +844,21 @@ k_density_walk(const uint2* __restrict__ tiles, uint32_t ntiles,
 // of each there for the first warp to sum in that order. The sums are therefore
 // the walk's bit for bit, while the chain a particle waits for is one row of
 // ~16 candidates instead of ~140 (measured: 16,384 particles 32 -> 11 us, 1,000
-// 39 -> 11 us). A particle with more hits than a queue or a list holds walks
-// all its rows again by itself. The 46 KB a block take the SM's occupancy, so
-// large launches lose (1M: 165 -> 292 us).
+// 39 -> 11 us). The 46 KB a block take the SM's occupancy, so large launches
+// lose (1M: 165 -> 292 us).
+//
+// Where a row has more hits than its queue holds, or the list overflows, the
+// warps walk their rows once more, now that the place of every hit is known, and
+// leave r - dist there themselves, past a list's length in the lane's queues. Only
+// a particle with more than kRowSums neighbours is walked by the first warp
+// alone. (Were it every such particle, one candidate at a time, a cloud of 60,000
+// particles took, density of a substep, us: at 45 / 100 / 200 / 400 neighbours 162 /
+// 310 / 584 / 1133, all particles at one point 51 ms; now 45 / 82 / 140 / 550, 13.4 ms;
+// k_density_walk with one candidate at a time 64 / 110 / 191 / 380, 9.6 ms.)
 constexpr int kRowWarps = 9;
 constexpr uint32_t kRowCap = 16;  // hits a queue holds
+constexpr uint32_t kRowSums = kNbrCap + 2u * kRowWarps * kRowCap;  // r - dist a lane has room for
+constexpr uint32_t kRowLong = 1024;  // a run of more candidates goes uncounted: more hits than that
 
 template <int kTables>
 __global__ void __launch_bounds__(32 * kRowWarps, 4)  // the blocks an SM's shared memory holds
@@ -826,81 +887,81 @@ k_density_rows(const uint2* __restrict__ tiles, uint32_t ntiles,
     const uint32_t cell = __float_as_uint(me.w);
     const uint32_t cf = kTables == kTablesDirect ? 0u : cell_first[i];
     const float2 npxy = make_float2(-me.x, -me.y);
-    uint32_t cnt = 0;
-    // four candidates at a time: their loads are in flight together (one at a
-    // time, prefetched, the row cost an L2 round trip a candidate)
-    auto run = [&](uint32_t j, uint32_t e) {
-      for (; j < e; j += 4u) {
-        float4 q[4];
-#pragma unroll
-        for (uint32_t u = 0; u < 4; ++u) q[u] = __ldg(pred + min(j + u, e - 1u));
-#pragma unroll
-        for (uint32_t u = 0; u < 4; ++u) {
-          const float2 dxy = __fadd2_rn(make_float2(q[u].x, q[u].y), npxy);
-          const float2 sxy = __fmul2_rn(dxy, dxy);
-          const float dz = q[u].z - me.z;
-          const float d2 = __fadd_rn(__fadd_rn(sxy.x, sxy.y), __fmul_rn(dz, dz));
-          if (j + u < e && d2 <= cut && j + u != i) {
-            if (cnt < kRowCap) s_hit[s][cnt][lane] = make_float2(d2, __uint_as_float(j + u));
-            ++cnt;
-          }
-        }
-      }
+    // the row's particles within the cutoff: hit(slot, distance squared)
+    auto row = [&](auto&& enter, auto&& hit) {
+      walk_row<kTables, 4>(direct, start, row0 + cell,
+                        cell_tab + static_cast<uint64_t>(cf) * 27u + s * 3u, pred, enter,
+                        [&](uint32_t j, float4 q, bool in) {
+        const float2 dxy = __fadd2_rn(make_float2(q.x, q.y), npxy);
+        const float2 sxy = __fmul2_rn(dxy, dxy);
+        const float dz = q.z - me.z;
+        const float d2 = __fadd_rn(__fadd_rn(sxy.x, sxy.y), __fmul_rn(dz, dz));
+        if (in && d2 <= cut && j != i) hit(j, d2);
+      });
     };
-    if (live) {
-      if (direct) {
-        const uint32_t k = row0 + cell;
-        run(__ldg(start + k - 1), __ldg(start + k + 2));
-      } else {
-        const uint2* tab = cell_tab + static_cast<uint64_t>(cf) * 27u + s * 3u;
-        const uint2 m = __ldg(tab);
-        if (m.y & kRunMerged) {
-          run(m.x, m.x + (m.y & ~kRunMerged));
-        } else {
-#pragma unroll 1
-          for (int k = 0; k < 3; ++k) {
-            const uint2 x = k ? __ldg(tab + k) : m;
-            run(x.x, x.x + x.y);
-          }
-        }
-      }
-    }
+    uint32_t cnt = 0;
+    if (live)
+      row([&](uint32_t len) {
+        if (len <= kRowLong) return true;
+        cnt = kRowSums + 1u;
+        return false;
+      }, [&](uint32_t j, float d2) {
+        if (cnt < kRowCap) s_hit[s][cnt][lane] = make_float2(d2, __uint_as_float(j));
+        ++cnt;
+      });
     s_cnt[s][lane] = cnt;
     __syncthreads();
     uint32_t before = 0, total = 0;
-    bool full = false;
 #pragma unroll
     for (uint32_t u = 0; u < kRowWarps; ++u) {
       const uint32_t c = s_cnt[u][lane];
       before += u < s ? c : 0u;
       total += c;
-      full |= c > kRowCap;
     }
-    full |= total > kNbrCap;
     uint32_t* const list = nbr + nbr_index(i, 0);
-    if (!full) {
+    // a term of the sums past a list's length: in the lane's queues, which
+    // nothing reads any more then
+    auto wide = [&](uint32_t k) -> float& {
+      const uint32_t q = k - kNbrCap;
+      return reinterpret_cast<float*>(&s_hit[0][0][lane])[q / 2u * 64u + q % 2u];
+    };
+    if (cnt <= kRowCap && total <= kNbrCap) {
       for (uint32_t k = 0; k < cnt; ++k) {
         const float2 h = s_hit[s][k][lane];
         s_w[before + k][lane] = r - sqrt_approx(h.x);
         list[(before + k) * 32u] = __float_as_uint(h.y);
       }
+    } else if (total <= kRowSums) {
+      uint32_t k = before;
+      row([](uint32_t) { return true; }, [&](uint32_t j, float d2) {
+        const float w = r - sqrt_approx(d2);
+        if (k < kNbrCap) {
+          s_w[k][lane] = w;
+          list[k * 32u] = j;
+        } else {
+          wide(k) = w;
+        }
+        ++k;
+      });
     }
     __syncthreads();
     if (s == 0 && live) {
       float s2 = S.r2, s3 = S.r2 * r;  // self: w = r
-      if (!full) {
+      if (total <= kRowSums) {
 #pragma unroll 4
-        for (uint32_t k = 0; k < total; ++k) density_sum(s_w[k][lane], s2, s3);
+        for (uint32_t k = 0; k < min(total, kNbrCap); ++k) density_sum(s_w[k][lane], s2, s3);
+#pragma unroll 4
+        for (uint32_t k = kNbrCap; k < total; ++k) density_sum(wide(k), s2, s3);
       } else {
         uint32_t k = 0;
-        walk_runs<kTables>(S, start, cell_tab, cf, cell, pred, [&](uint32_t j, float4 q) {
+        walk_rows<kTables, 4>(S, start, cell_tab, cf, cell, pred, [&](uint32_t j, float4 q, bool in) {
           const float d2 = dist2(q.x - me.x, q.y - me.y, q.z - me.z);
-          if (d2 <= cut && j != i) {
-            if (k < kNbrCap) list[k * 32u] = j;
-            ++k;
-            density_sum(r - sqrt_approx(d2), s2, s3);
-          }
+          const bool hit = in && d2 <= cut && j != i;
+          if (hit && k < kNbrCap) list[k * 32u] = j;
+          k += hit;
+          density_sum(hit ? r - sqrt_approx(d2) : 0.0f, s2, s3);  // + 0: no branch to wait in
         });
+        total = k;
       }
       density_store(S, i, s2, s3, total, dens_a, dens_b, ncount);
     }
@@ -1168,7 +1229,10 @@ __global__ void k_pressure(const uint2* __restrict__ tiles, uint32_t ntiles,
 // with the operations of pressure_pair, so the result is k_pressure's bit for bit
 // (16,384 particles 14 -> 10 us; with 8 instead of 32 particles a warp and the
 // terms staged it takes 2.3 times the plain form's instructions, which large
-// launches pay: 1M 93 -> 210 us).
+// launches pay: 1M 93 -> 210 us). A list that overflowed goes by walk_rows, two
+// candidates in flight here (four spill) and four in the viscosity pass (a cloud
+// of 28,000 particles of 200 neighbours, pressure / viscosity, us: one in flight
+// 372 / 408, now 340 / 289, the plain forms 300 / 287).
 constexpr int kCoopTerms = kNbrCap + 1;  // float4 rows, shifted a bank group each
 constexpr int kCoopGather = 8;           // entries a lane has in flight (4: 16k-particle step 3 us longer)
 
@@ -1236,9 +1300,9 @@ k_pressure_coop(const uint2* __restrict__ tiles, uint32_t ntiles,
         }
       }
     } else if (part == 0) {
-      walk_runs<kTables>(S, start, cell_tab, cell_first[i], __float_as_uint(pi.w), pred,
-                         [&](uint32_t j, float4 q) {
-        if (j == i) return;
+      walk_rows<kTables, 2>(S, start, cell_tab, cell_first[i], __float_as_uint(pi.w), pred,
+                         [&](uint32_t j, float4 q, bool in) {
+        if (!in || j == i) return;
         const float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
         if (dist2(dx, dy, dz) <= S.cut_le)
           pressure_pair(S, p, Pi, Pni, q, __ldg(dens_b + j), f);
@@ -1479,9 +1543,9 @@ __global__ void __launch_bounds__(kCoopBlock) k_visc_coop(
         }
       }
     } else if (part == 0) {
-      walk_runs<kTables>(S, start, cell_tab, cell_first[i], __float_as_uint(pi.w), pred,
-                         [&](uint32_t j, float4 q) {
-        if (j != i) visc_pair(S, p, vi, q, __ldg(rec_v + 2ull * j + 1), f);
+      walk_rows<kTables, 4>(S, start, cell_tab, cell_first[i], __float_as_uint(pi.w), pred,
+                         [&](uint32_t j, float4 q, bool in) {
+        if (in && j != i) visc_pair(S, p, vi, q, __ldg(rec_v + 2ull * j + 1), f);
       });
     }
     __syncwarp();
