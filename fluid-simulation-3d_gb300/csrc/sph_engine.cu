@@ -531,6 +531,8 @@ int Engine::RunSubsteps(int substeps, cudaStream_t st, bool carry) {
   c.tables = tables_;
   c.pdl = !profile_;  // phase events between kernels need plain launches
   c.max_blocks = 0;
+  c.particles = total_;
+  c.live = NumScenes();
   c.src_limit = static_cast<uint32_t>(capacity_);
   int cur = cur_;
   const Tiles told{d_tiles_old_, n_tiles_old_};

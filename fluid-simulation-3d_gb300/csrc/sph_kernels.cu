@@ -732,7 +732,7 @@ __device__ __forceinline__ void density_store(const SceneDev& S, uint32_t i,
 // Thread-per-particle form in one pass: each lane walks its cell's runs,
 // classifies every candidate on the reference's exact d2 and accumulates the
 // density and its list as it goes. Lanes of one cell walk identical runs, so
-// their loads coincide; a lane keeps kWalkBatch candidates in flight (the loads of a
+// their loads coincide; a lane keeps kBatch candidates in flight (the loads of a
 // run's last batch may pass its end by kPredPad slots, whose pairs are
 // dropped). At large sizes it fills 78% of the issue slots and 70% of the L1 data
 // pipe (26 warp instructions a candidate, of which the hit path takes a third;
@@ -740,10 +740,11 @@ __device__ __forceinline__ void density_store(const SceneDev& S, uint32_t i,
 // time at 32 registers: 131k particles 37 -> 30 us (a step of three substeps
 // 298 -> 248), 500k 93 -> 84, 1M 166 -> 157, 4M 581 -> 567, 8.4M 1149 -> 1161.
 // Batches of 2, 3, 5, 6, 8 and caps of 32, 36, 40 registers (spills) were slower.
-constexpr int kWalkBatch = 4;
-static_assert(kWalkBatch - 1 <= static_cast<int>(kPredPad), "candidate loads past the last slot");
+// Batches of tiny scenes keep one candidate at 32 registers (tiny_scenes).
+constexpr uint32_t kWalkBatch = 4;
+static_assert(kWalkBatch - 1u <= kPredPad, "candidate loads past the last slot");
 
-template <int kTables, int kRegs>
+template <int kTables, int kRegs, uint32_t kBatch>
 __global__ void __maxnreg__(kRegs)
 k_density_walk(const uint2* __restrict__ tiles, uint32_t ntiles,
                 const SceneDev* __restrict__ scenes, const float4* __restrict__ pred,
@@ -773,12 +774,12 @@ k_density_walk(const uint2* __restrict__ tiles, uint32_t ntiles,
     uint32_t* wp = nbr + nbr_index(i, 0);
     auto run = [&](uint32_t j, uint32_t e) {
 #pragma unroll 1
-      for (; j < e; j += kWalkBatch) {
-        float4 q[kWalkBatch];
+      for (; j < e; j += kBatch) {
+        float4 q[kBatch];
 #pragma unroll
-        for (uint32_t u = 0; u < kWalkBatch; ++u) q[u] = __ldg(pred + j + u);
+        for (uint32_t u = 0; u < kBatch; ++u) q[u] = __ldg(pred + j + u);
 #pragma unroll
-        for (uint32_t u = 0; u < kWalkBatch; ++u) {
+        for (uint32_t u = 0; u < kBatch; ++u) {
           // dist2 with (dx, dy) as one packed FP32x2 pair (x and y are
           // adjacent in the record), every component rounded as the scalar
           // code rounds it
@@ -1990,11 +1991,29 @@ uint32_t scan_partials_needed(uint64_t len) {
 // particle, the cell tile) keep their own kernels.
 constexpr uint32_t kRowsTiles = 2048;  // 65,536 particles
 constexpr uint32_t kCoopTiles = 900;   // 28,800 particles
+
+// Batches of tiny scenes: a tile each, mostly empty, whose walks are over after a
+// few candidates. There the number of tiles at work counts: the latency forms
+// hold four an SM and are kept to one wave of those, and the walk runs at 32
+// registers (64 tiles an SM), a candidate at a time. Substeps of scenes x
+// particles, us, by the other launches' forms / by these: 2,048 x 1 27.0 / 20.7,
+// 2,000 x 9 34.1 / 31.0, 2,000 x 16 39.1 / 38.0, 16,000 x 3 54.7 / 49.3, 30,000 x 2
+// 74.9 / 67.8, 16,000 x 10 79.7 / 74.4; but 2,000 x 24 43.3 / 45.0, 1,000 x 33
+// 50.0 / 59.6.
+constexpr uint32_t kTinyScene = 20;    // particles, on average
+constexpr uint32_t kLatencyTiles = 4;  // tiles an SM holds in the latency forms
+bool tiny_scenes(const LaunchCtx& c) { return c.particles < uint64_t{kTinyScene} * c.live; }
+bool latency_wave(const LaunchCtx& c, uint32_t ntiles) {
+  return !tiny_scenes(c) || ntiles <= kLatencyTiles * c.sms;
+}
+bool rows_table(const LaunchCtx& c, uint32_t ntiles) {
+  return ntiles <= kRowsTiles && latency_wave(c, ntiles);
+}
 bool rows_form(const LaunchCtx& c, uint32_t ntiles) {
-  return c.cell_tile <= 1 && ntiles <= kRowsTiles;
+  return c.cell_tile <= 1 && rows_table(c, ntiles);
 }
 bool coop_form(const LaunchCtx& c, uint32_t ntiles) {
-  return c.lanes == 1 && ntiles <= kCoopTiles;
+  return c.lanes == 1 && ntiles <= kCoopTiles && latency_wave(c, ntiles);
 }
 
 // Launches whose plain neighbour kernels fit the GPU in about one wave (48
@@ -2074,7 +2093,7 @@ cudaError_t launch_sort_reorder(const LaunchCtx& c, const Tiles& old_tiles,
                    c.tmp_src, c.start, c.pos, c.vel, c.pos2, c.vel2, c.pred,
                    c.hash_s, c.cell_first, c.src_limit, c.status);
     if (e == cudaSuccess && c.tables != kTablesDirect)
-      e = new_tiles.n <= kRowsTiles
+      e = rows_table(c, new_tiles.n)
               ? launch_pdl(c.pdl, k_cell_table_rows, new_tiles.n, 32 * kRowWarps, st, new_tiles.d,
                            new_tiles.n, c.scenes, c.hash_s, c.cell_first, c.start, c.cell_tab)
               : launch_pdl(c.pdl, k_cell_table,
@@ -2085,10 +2104,10 @@ cudaError_t launch_sort_reorder(const LaunchCtx& c, const Tiles& old_tiles,
   return e;
 }
 
-template <int kRegs> auto density_kernel(int tables) {
-  return tables == kTablesDirect    ? k_density_walk<kTablesDirect, kRegs>
-         : tables == kTablesBuckets ? k_density_walk<kTablesBuckets, kRegs>
-                                    : k_density_walk<kTablesMixed, kRegs>;
+template <int kRegs, uint32_t kBatch> auto density_kernel(int tables) {
+  return tables == kTablesDirect    ? k_density_walk<kTablesDirect, kRegs, kBatch>
+         : tables == kTablesBuckets ? k_density_walk<kTablesBuckets, kRegs, kBatch>
+                                    : k_density_walk<kTablesMixed, kRegs, kBatch>;
 }
 
 cudaError_t launch_density(const LaunchCtx& c, const Tiles& tiles,
@@ -2105,8 +2124,9 @@ cudaError_t launch_density(const LaunchCtx& c, const Tiles& tiles,
   const uint32_t g = grid_for(tiles.n, b, c.max_blocks);
   if (c.cell_tile <= 1)
     return launch_pdl(c.pdl && !one_wave(c, tiles.n),
-                      dense_wave(c, tiles.n) ? density_kernel<40>(c.tables)
-                                             : density_kernel<48>(c.tables),
+                      tiny_scenes(c)           ? density_kernel<32, 1>(c.tables)
+                      : dense_wave(c, tiles.n) ? density_kernel<40, kWalkBatch>(c.tables)
+                                               : density_kernel<48, kWalkBatch>(c.tables),
                       g, b, st, tiles.d, tiles.n, c.scenes, c.pred,
                       c.start, c.cell_first, c.cell_tab, c.dens_a, c.dens_b, c.nbr,
                       c.ncount, 32u, kNbrCap);

@@ -85,6 +85,8 @@ struct LaunchCtx {
   uint2* dbg_keyrank = nullptr;     // (key, arrival rank) per slot
   uint32_t* dbg_tmp = nullptr;      // bucketed particle indices
   uint32_t* dbg_sorted = nullptr;   // (key, index)-ordered particle indices
+  uint32_t particles = 0;  // of all scenes
+  uint32_t live = 0;       // scenes
   uint32_t src_limit = 0;  // slots of the layout a substep reads
   bool pdl = true;        // programmatic dependent launch (off while the
                           // engine records phase events between kernels)
