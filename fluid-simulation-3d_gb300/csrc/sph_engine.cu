@@ -3,6 +3,7 @@
 #include "sph_render.h"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -519,9 +520,8 @@ int Engine::UploadScenes(int substeps, cudaStream_t st) {
   return SPH_OK;
 }
 
-// Launches `substeps` substeps starting from state buffers cur_. Does not
-// change engine state, so it can run under stream capture.
-int Engine::RunSubsteps(int substeps, cudaStream_t st, bool carry) {
+// The launch context under the current tuning.
+LaunchCtx Engine::Context() const {
   LaunchCtx c = ctx_;
   c.block_nbr = tuning_.block;
   c.block_force = tuning_.force_block ? tuning_.force_block : tuning_.block;
@@ -534,6 +534,13 @@ int Engine::RunSubsteps(int substeps, cudaStream_t st, bool carry) {
   c.particles = total_;
   c.live = NumScenes();
   c.src_limit = static_cast<uint32_t>(capacity_);
+  return c;
+}
+
+// Launches `substeps` substeps starting from state buffers cur_. Does not
+// change engine state, so it can run under stream capture.
+int Engine::RunSubsteps(int substeps, cudaStream_t st, bool carry) {
+  LaunchCtx c = Context();
   int cur = cur_;
   const Tiles told{d_tiles_old_, n_tiles_old_};
   const Tiles tnew{d_tiles_new_, n_tiles_new_};
@@ -974,9 +981,12 @@ int Engine::SetTuning(const sph_tuning& t) {
   return SPH_OK;
 }
 
-// Coordinate search: block size x cell tile (all neighbour kernels), then
-// the block size of the force kernels alone, then their particles per warp x
-// gather batch.
+// Coordinate search from the current tuning: block size x cell tile (all
+// neighbour kernels), then the block size of the force kernels alone, then their
+// particles per warp x gather batch. Settings that launch the kernels of one
+// already timed (small launches choose blocks and batches themselves) are left
+// out: which of them was faster would be chance, and the one kept would later
+// count in a larger launch.
 int Engine::Autotune(int substeps, int steps_per_trial, sph_tuning* best,
                      float* best_ms, cudaStream_t st) {
   if (steps_per_trial < 1) return Fail(SPH_ERR_INVALID, "steps_per_trial >= 1");
@@ -1026,13 +1036,16 @@ int Engine::Autotune(int substeps, int steps_per_trial, sph_tuning* best,
   cudaEvent_t e0 = ev.e0, e1 = ev.e1;
   const int ppw0 = tuning_.particles_per_warp;
   int rc = SPH_OK;
-  for (int round = 0; round < 3 && rc == SPH_OK; ++round) {
+  std::vector<std::array<int, 8>> timed;
+  for (int round = 0; round < 4 && rc == SPH_OK; ++round) {
     std::vector<sph_tuning> space;
     if (round == 0) {
+      space.push_back(tuning_);
+    } else if (round == 1) {
       for (int b : {64, 128, 256, 512})
         for (int tile : {1, 64, 128, 256})
           space.push_back(sph_tuning{b, tile, ppw0, tuning_.gather, 0, tuning_.table});
-    } else if (round == 1) {
+    } else if (round == 2) {
       for (int fb : {64, 128, 256, 512})
         space.push_back(sph_tuning{win.block, win.cell_tile, win.particles_per_warp,
                                    win.gather, fb, win.table});
@@ -1040,13 +1053,23 @@ int Engine::Autotune(int substeps, int steps_per_trial, sph_tuning* best,
       // the force kernels' mapping: particles per warp (one or two lanes a
       // particle) x gather batch
       for (int ppw : {32, 16})
-        for (int g : {2, 3, 4, 8})
+        for (int g : {win.gather, 2, 3, 4, 8})
           space.push_back(sph_tuning{win.block, win.cell_tile, ppw, g, win.force_block,
                                      win.table});
     }
     for (const sph_tuning& t : space) {
       if ((rc = SetTuning(t)) != SPH_OK) break;
-      if ((rc = Step(substeps, st)) != SPH_OK) break;  // warm-up + capture
+      if (round > 0 && std::find(timed.begin(), timed.end(),
+                                 launch_forms(Context(), n_tiles_new_)) != timed.end())
+        continue;
+      rc = Step(substeps, st);  // warm-up + capture
+      if (rc != SPH_OK && round == 0) {
+        cudaGetLastError();  // a tuning whose blocks no kernel fits: the sweep goes on
+        rc = SPH_OK;
+        continue;
+      }
+      if (rc != SPH_OK) break;
+      timed.push_back(launch_forms(Context(), n_tiles_new_));
       cudaEventRecord(e0, st);
       for (int k = 0; k < steps_per_trial && rc == SPH_OK; ++k) rc = Step(substeps, st);
       cudaEventRecord(e1, st);

@@ -101,6 +101,7 @@ class Engine {
   };
   int BuildLayout(cudaStream_t st);
   int UploadScenes(int substeps, cudaStream_t st);
+  LaunchCtx Context() const;
   int RunSubsteps(int substeps, cudaStream_t st, bool carry);
   int RefuseCapture(cudaStream_t st);
   void ReleaseGraphs();

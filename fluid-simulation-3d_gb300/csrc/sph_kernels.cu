@@ -32,6 +32,7 @@
 #include "sph_kernels.h"
 
 #include <algorithm>
+#include <array>
 
 namespace sph {
 
@@ -2074,6 +2075,18 @@ int force_gather(const LaunchCtx& c, uint32_t ntiles) {
                      ntiles <= kDenseWaves * kWaveWarps * c.sms &&
                      waves(c, ntiles, kGather3Warps) == waves(c, ntiles, kWaveWarps);
   return std::max(c.gather, ntiles <= kGather8Tiles ? 8 : ntiles <= kRowsTiles ? 4 : three ? 3 : 2);
+}
+
+std::array<int, 8> launch_forms(const LaunchCtx& c, uint32_t ntiles) {
+  const bool rows = rows_form(c, ntiles), coop = coop_form(c, ntiles);
+  return {c.cell_tile,
+          rows ? 0 : c.block_nbr,
+          rows ? 0 : dense_wave(c, ntiles),
+          coop ? 0 : c.lanes,
+          coop ? 0 : c.block_force,
+          coop ? 0 : force_gather(c, ntiles),
+          coop ? 0 : dense_form(c, ntiles),
+          one_wave(c, ntiles)};
 }
 
 cudaError_t launch_sort_reorder(const LaunchCtx& c, const Tiles& old_tiles,

@@ -1,6 +1,7 @@
 // Host-visible declarations of the SPH kernels' launchers.
 #pragma once
 
+#include <array>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -120,6 +121,9 @@ cudaError_t launch_scan(const LaunchCtx& c, uint32_t len, cudaStream_t st);
 cudaError_t launch_sort_reorder(const LaunchCtx& c, const Tiles& old_tiles,
                                 const Tiles& new_tiles, uint32_t total,
                                 cudaStream_t st);
+// What the neighbour kernels of a launch depend on, out of its tuning: equal for
+// two tunings that launch the same kernels in the same blocks.
+std::array<int, 8> launch_forms(const LaunchCtx& c, uint32_t ntiles);
 cudaError_t launch_density(const LaunchCtx& c, const Tiles& tiles,
                            cudaStream_t st);
 cudaError_t launch_pressure(const LaunchCtx& c, const Tiles& tiles,

@@ -65,7 +65,11 @@ typedef struct sph_sim sph_sim;
  * (sph_autotune / sph_batch_autotune) by timing real steps. */
 typedef struct sph_tuning {
   int32_t block;      /* threads per block of the neighbour kernels
-                         (multiple of 32, 32..1024), default 128          */
+                         (multiple of 32, 32..1024), default 128; small
+                         launches take kernels with blocks of their own:
+                         up to 65,536 particles (2,048 tiles of 32) the
+                         density pass, up to 28,800 (900 tiles) also the
+                         other two with particles_per_warp = 32          */
   int32_t cell_tile;  /* density kernel: 1 = one lane per particle walking
                          its cell's runs (default); 64, 128, 192 or 256 =
                          warp-cooperative form holding that many candidates
@@ -77,10 +81,12 @@ typedef struct sph_tuning {
   int32_t gather;     /* neighbour-list entries whose gathers the force
                          kernels issue together: 2, 3, 4 or 8 (default 2;
                          small launches issue 4 or 8 at least, some of a
-                         few waves 3, in blocks of up to 512). Results do
-                         not depend on it                                 */
+                         few waves 3, in blocks of up to 512, and fewer
+                         where the block leaves too few registers).
+                         Results do not depend on it                     */
   int32_t force_block; /* threads per block of the pressure and viscosity
-                          kernels (multiple of 32, 32..1024); 0 = block   */
+                          kernels (multiple of 32, 32..1024); 0 = block;
+                          small launches as for block                    */
   int32_t table;      /* key table of the sort: 0 = one entry per cell of
                          the scene's grid where the grid has at most four
                          cells per particle, else n entries (cell index
@@ -235,10 +241,11 @@ int sph_phase_times(sph_sim *sim, double out_ms[6]);
 
 /* Kernel launch configuration of a single-scene handle, and its autotuner:
  * times real steps of dt/substeps (steps_per_trial per candidate, after one
- * untimed step) over the neighbour block size x cell tile, then the force
- * kernels' block size, then their particles per warp x gather batch; keeps
- * the fastest and reports
- * it (best may be NULL) with its ms per step. The state (positions,
+ * untimed step) under the current tuning, then over the neighbour block size x
+ * cell tile, the force kernels' block size, and their particles per warp x
+ * gather batch; keeps the fastest and reports it (best may be NULL) with its
+ * ms per step. Settings that make no difference to a launch of this size keep
+ * the value they have. The state (positions,
  * velocities, densities, OutPositions) is saved before the sweep and
  * restored after it. */
 int sph_set_tuning(sph_sim *sim, const sph_tuning *t);
