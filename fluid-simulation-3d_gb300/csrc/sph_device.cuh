@@ -77,7 +77,6 @@ struct SceneDev {
   float cut_lo;       // cut_lt narrowed by 2e-6: an FMA estimate below it
                       // certifies d2 <= cut_lt without the exact recompute
   float r2;           // r*r
-  float inv_r;        // 1/r
   float vol2, vol3;   // density kernel scales   (kernels.h:28,40)
   float ds2h, ds3h;   // 0.5 * derivative scales (kernels.h:52,64)
   float vscale;       // poly6 scale             (kernels.h:76)

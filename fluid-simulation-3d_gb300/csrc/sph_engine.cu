@@ -114,7 +114,6 @@ SceneDev MakeSceneDev(const sph_params& p, uint32_t n, uint32_t base, uint32_t t
   d.cut_hi = d.cut_le * 1.000002f;
   d.cut_lo = d.cut_lt * 0.999998f;
   d.r2 = r * r;
-  d.inv_r = 1.0f / r;
   // kernels.h:28,40,52,64,76 -- same float expressions.
   d.vol2 = 15.0f / (2.0f * kPiF * powf(r, 5.0f));
   d.vol3 = 15.0f / (kPiF * powf(r, 6.0f));

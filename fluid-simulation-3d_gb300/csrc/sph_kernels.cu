@@ -1899,12 +1899,12 @@ k_import_rows(uint32_t first, uint32_t n, const float* __restrict__ ipos,
 // pdl_wait(), which hides the launch and ramp-up between the seven to nine
 // kernels of a substep (inside a graph these become programmatic edges).
 template <class... KArgs, class... Args>
-cudaError_t launch_pdl_smem(bool pdl, void (*kernel)(KArgs...), uint32_t grid, int block,
-                            size_t smem, cudaStream_t st, Args... args) {
+cudaError_t launch_pdl(bool pdl, void (*kernel)(KArgs...), uint32_t grid, int block,
+                       cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(static_cast<unsigned>(block));
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = 0;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1912,12 +1912,6 @@ cudaError_t launch_pdl_smem(bool pdl, void (*kernel)(KArgs...), uint32_t grid, i
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-
-template <class... KArgs, class... Args>
-cudaError_t launch_pdl(bool pdl, void (*kernel)(KArgs...), uint32_t grid, int block,
-                       cudaStream_t st, Args... args) {
-  return launch_pdl_smem(pdl, kernel, grid, block, 0, st, args...);
 }
 
 template <int N>
