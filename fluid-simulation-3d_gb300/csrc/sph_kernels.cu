@@ -58,11 +58,11 @@ __device__ __forceinline__ float dist2(float dx, float dy, float dz) {
 __device__ __forceinline__ float dist2_fast(float dx, float dy, float dz) {
   return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
 }
-// Hardware square root estimate (0 -> 0). Flushing denormals saves the walk
-// the range test and the two scalings of the plain form (172 -> 164 us at 1M,
-// 1204 -> 1140 us at 8.4M) and changes no density: the result is only used as
-// r - sqrt(d2), a denormal d2 has sqrt(d2) < 1.1e-19, and r - 1.1e-19 rounds
-// to r for every radius whose 1/r^5 kernel scale is finite.
+// Hardware square root estimate (0 -> 0). The form that flushes denormals is
+// faster (walk 172 -> 164 us at 1M, 1204 -> 1140 us at 8.4M) and changes no
+// density: the result is only used as r - sqrt(d2), a denormal d2 has sqrt(d2) <
+// 1.1e-19, and r - 1.1e-19 rounds to r for every radius whose 1/r^5 kernel scale
+// is finite.
 __device__ __forceinline__ float sqrt_approx(float x) {
   float y;
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -698,13 +698,11 @@ k_cell_table_rows(const uint2* __restrict__ tiles, uint32_t ntiles,
 
 // ----------------------------------------------------------------- density
 // CalculateDensity (:325-365) for one particle (self included) and its
-// neighbour list (dist <= r, self excluded) for the force passes, in two
-// phases. Phase 1 walks the cell's runs with the FMA estimate of d2 and only
-// appends candidates within cut_hi (a 2e-6 superset of the cutoff) to the
-// list. Phase 2 re-reads the ~25 listed pairs, classifies each on the
-// reference's exact d2 (dropping the rare band pairs) and accumulates the
-// kernels; contributions vanish at the cutoff ((r-dist)^2), so the hardware
-// square root serves the kernel value. The self pair contributes (r, r).
+// neighbour list (dist <= r, self excluded) for the force passes. The walk forms
+// classify every candidate on the reference's exact d2 and sum as they go; the
+// cell-tile form lists by an estimate first (k_density). Contributions vanish at
+// the cutoff ((r-dist)^2), so the hardware square root serves the kernel value.
+// The self pair contributes (r, r).
 // One pair's share of the density sums, w = r - dist.
 __device__ __forceinline__ void density_sum(float w, float& s2, float& s3) {
   const float w2 = w * w;
@@ -769,9 +767,8 @@ k_density_walk(const uint2* __restrict__ tiles, uint32_t ntiles,
     float s2 = S.r2, s3 = S.r2 * r;  // self: w = r
     uint32_t cnt = 0;
     // next list entry: a bumped pointer is the cheapest append in the hit
-    // path, and it stays one only while the step and the capacity are
-    // run-time values (with constants the compiler recomputes the address
-    // from cnt: 195 instead of 172 us at 1M)
+    // path. The step and the capacity are run-time values: with constants in
+    // their place the kernel takes 195 instead of 172 us at 1M
     uint32_t* wp = nbr + nbr_index(i, 0);
     auto run = [&](uint32_t j, uint32_t e) {
 #pragma unroll 1
@@ -977,6 +974,9 @@ constexpr int kCoopSub = kTile / kCoopPer;  // warps a tile
 constexpr int kCoopBlock = 128;
 constexpr int kCoopWarps = kCoopBlock / 32;
 
+// Cell-tile form, in two phases. Phase 1 lists the candidates within cut_hi, a
+// 2e-6 superset of the cutoff, by the FMA estimate of d2; phase 2 re-reads the
+// listed pairs, classifies each on the exact d2 and sums.
 // Phase 1 is warp-cooperative over the cells of the warp's 32 slots: for
 // each cell, lanes 0..26 fetch its 27 runs, a warp scan gives their offsets
 // in the cell's flat candidate sequence, and each lane holds kChunks of those

@@ -282,8 +282,9 @@ const char *sph_global_error(void);
  * allocating library call. The first call on a device resolves that array's
  * address (cudaGetSymbolAddress) with the device current, so make the first
  * call on each device before any stream capture. Each device has its own
- * copy of the array and every call on that device shares it, keeping the
- * last call's contents (each call clears what must start at zero): two calls
+ * copy of the array and every call on that device shares it (it holds the
+ * entries between the call's two sorting passes, written before they are
+ * read, so nothing needs clearing): two calls
  * whose work overlaps on the same GPU, e.g. on different streams, race, so
  * serialise them (one stream does). Asynchronous on `stream`; the message of
  * the last failure is sph_static_error(). */
