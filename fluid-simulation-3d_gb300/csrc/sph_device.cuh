@@ -194,4 +194,27 @@ __device__ __forceinline__ uint32_t pdl_enter(uint32_t x) {
   return pdl_wait(x);
 }
 
+// Launches. Substep kernels go out with programmatic stream serialisation
+// (pdl): the next kernel is scheduled during its predecessor's last wave and
+// waits for it in pdl_wait(), which hides the launch and ramp-up between the
+// seven to nine kernels of a substep (inside a graph these become programmatic
+// edges). The result is this launch's own: an error that an earlier call of the
+// library or of its caller left behind is not taken for it, as it would be if
+// cudaGetLastError were asked.
+template <class... KArgs, class... Args>
+cudaError_t launch_pdl(bool pdl, void (*kernel)(KArgs...), uint32_t grid, int block,
+                       cudaStream_t st, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(static_cast<unsigned>(block));
+  cfg.dynamicSmemBytes = 0;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 }  // namespace sph

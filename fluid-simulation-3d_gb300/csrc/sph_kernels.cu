@@ -1894,34 +1894,14 @@ k_import_rows(uint32_t first, uint32_t n, const float* __restrict__ ipos,
 }  // namespace
 
 // ------------------------------------------------------------- launchers
-// Substep kernels go out with programmatic stream serialisation: the next
-// kernel is scheduled during its predecessor's last wave and waits for it in
-// pdl_wait(), which hides the launch and ramp-up between the seven to nine
-// kernels of a substep (inside a graph these become programmatic edges).
-template <class... KArgs, class... Args>
-cudaError_t launch_pdl(bool pdl, void (*kernel)(KArgs...), uint32_t grid, int block,
-                       cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(static_cast<unsigned>(block));
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-
 template <int N>
 cudaError_t launch_scene_chunk(SceneDev* table, const SceneDev* host, uint32_t count,
                                cudaStream_t st) {
   SceneChunk<N> chunk;
   std::copy(host, host + count, chunk.s);
-  k_scenes<N><<<1, 256, 0, st>>>(chunk, count * static_cast<uint32_t>(sizeof(SceneDev) / 4),
-                                 reinterpret_cast<uint32_t*>(table));
-  return cudaGetLastError();
+  return launch_pdl(false, k_scenes<N>, 1, 256, st, chunk,
+                    count * static_cast<uint32_t>(sizeof(SceneDev) / 4),
+                    reinterpret_cast<uint32_t*>(table));
 }
 
 cudaError_t launch_scenes(SceneDev* scene_table, const SceneDev* host, uint32_t scenes,
@@ -2250,17 +2230,16 @@ cudaError_t launch_export(uint32_t first, uint32_t n, const float4* pos,
                           float* ovel, float* odens, uint32_t* oids,
                           cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  k_export<<<(n + 255) / 256, 256, 0, st>>>(first, n, pos, vel, dens, opos,
-                                            ovel, odens, oids);
-  return cudaGetLastError();
+  return launch_pdl(false, k_export, (n + 255) / 256, 256, st, first, n, pos, vel, dens, opos,
+                    ovel, odens, oids);
 }
 
 cudaError_t launch_export_rows(uint32_t first, uint32_t n, const float4* pos,
                               const float4* vel, const float2* dens, uint32_t* slot_of,
                               float* opos, float* ovel, float* odens, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  k_slot_map<<<(n + 255) / 256, 256, 0, st>>>(first, n, pos, slot_of);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e =
+      launch_pdl(false, k_slot_map, (n + 255) / 256, 256, st, first, n, pos, slot_of);
   if (e != cudaSuccess) return e;
   return launch_pdl(true, k_export_rows, (n + 255) / 256, 256, st, first, n, slot_of, pos, vel,
                     dens, opos, ovel, odens);
@@ -2271,18 +2250,16 @@ cudaError_t launch_export_debug(uint32_t first, uint32_t n, const float4* pos,
                                 const float4* velv, float* oaccp, float* ovelp,
                                 float* ovelv, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  k_export_debug<<<(n + 255) / 256, 256, 0, st>>>(first, n, pos, accp, velp,
-                                                  velv, oaccp, ovelp, ovelv);
-  return cudaGetLastError();
+  return launch_pdl(false, k_export_debug, (n + 255) / 256, 256, st, first, n, pos, accp, velp,
+                    velv, oaccp, ovelp, ovelv);
 }
 
 cudaError_t launch_export_layout(uint32_t first, uint32_t n, const SceneDev* scene,
                                  const float4* pos, const float4* pred, uint32_t* ocell,
                                  uint32_t* okey, uint32_t* oslot, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  k_export_layout<<<(n + 255) / 256, 256, 0, st>>>(first, n, scene, pos, pred, ocell,
-                                                  okey, oslot);
-  return cudaGetLastError();
+  return launch_pdl(false, k_export_layout, (n + 255) / 256, 256, st, first, n, scene, pos, pred,
+                    ocell, okey, oslot);
 }
 
 cudaError_t launch_ref_lookup(const LaunchCtx& c, const Tiles& new_tiles,
@@ -2310,8 +2287,8 @@ cudaError_t launch_import(uint32_t first, uint32_t n, const float* ipos,
                           const float* ivel, float4* pos, float4* vel, float2* dens,
                           cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  k_import<<<(n + 255) / 256, 256, 0, st>>>(first, n, ipos, ivel, pos, vel, dens);
-  return cudaGetLastError();
+  return launch_pdl(false, k_import, (n + 255) / 256, 256, st, first, n, ipos, ivel, pos, vel,
+                    dens);
 }
 
 cudaError_t launch_import_rows(uint32_t first, uint32_t n, const float* ipos,
@@ -2323,8 +2300,8 @@ cudaError_t launch_import_rows(uint32_t first, uint32_t n, const float* ipos,
   const bool beside = words && n > kClearRows;
   cudaError_t e = cudaSuccess;
   if (beside) {
-    k_clear<<<(words + 255) / 256, 256, 0, st>>>(reinterpret_cast<uint4*>(count), words);
-    e = cudaGetLastError();
+    e = launch_pdl(false, k_clear, (words + 255) / 256, 256, st, reinterpret_cast<uint4*>(count),
+                   words);
   } else if (words) {
     e = cudaMemsetAsync(count, 0, sizeof(uint4) * words, st);
   }

@@ -260,20 +260,13 @@ cudaError_t launch_render(uint32_t first, uint32_t n, const float4* pos, const f
                 : sub == 2 ? k_splat<2>
                            : k_splat<1>;
     const uint32_t per = 256u / static_cast<uint32_t>(sub);
-    kern<<<(n + per - 1) / per, 256, 0, st>>>(first, n, pos, vel, view, keys, colours);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = launch_pdl(false, kern, (n + per - 1) / per, 256, st, first, n, pos, vel, view, keys,
+                   colours);
+    if (e != cudaSuccess) return e;
   }
   const uint32_t px = view.width * view.height;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((px + 1023) / 1024);
-  cfg.blockDim = dim3(256);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = n ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, k_resolve, px, keys, colours, view.clear, rgba, depth);
+  return launch_pdl(n != 0, k_resolve, (px + 1023) / 1024, 256, st, px, keys, colours, view.clear,
+                    rgba, depth);
 }
 
 }  // namespace sph

@@ -236,9 +236,8 @@ extern "C" int sph_spatial_lookup_static(const float* dpred3, uint32_t n,
     scratch = g_scratch_addr[dev];
   }
   const uint64_t fm = (~static_cast<uint64_t>(0)) / n + 1;
-  k_lookup_static<<<kBlocks, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      dpred3, n, radius, fm, scratch, dhash, dkey, dsorted_ids, dstart);
-  e = cudaGetLastError();
+  e = launch_pdl(false, k_lookup_static, kBlocks, kThreads, static_cast<cudaStream_t>(stream),
+                 dpred3, n, radius, fm, scratch, dhash, dkey, dsorted_ids, dstart);
   if (e != cudaSuccess)
     return fail(SPH_ERR_CUDA, std::string("lookup kernel: ") + cudaGetErrorString(e));
   return SPH_OK;
