@@ -16,7 +16,8 @@
 // kernel of one eight-block cluster whose work is linear in n whatever the
 // keys: a stable radix sort of the 16-bit keys in two passes of 8 bits, so a
 // scene whose particles all share one key costs what any other scene of its
-// size does.
+// size does. (Up to 512 particles one block ranks every entry among the others,
+// without the working memory; that cost depends on n alone, too.)
 #include <cstdint>
 #include <mutex>
 #include <string>
@@ -186,6 +187,46 @@ k_lookup_static(const float* __restrict__ pred3, uint32_t n, float r,
   }
 }
 
+// The smallest calls: one block of a thread a particle, which ranks its entry
+// among all of them. A cluster's launch and barriers would be most of such a call.
+// us a call, the cluster / this: 32 particles 8.4 / 4.3, 100 8.4 / 4.2, 256 10.0 /
+// 4.3, 400 10.4 / 6.4, 512 10.4 / 8.4; the ranking grows with n^2, so the line is
+// drawn there.
+constexpr uint32_t kSmall = 512;
+__global__ void __launch_bounds__(kSmall)
+k_lookup_small(const float* __restrict__ pred3, uint32_t n, float r, uint64_t fm,
+               uint32_t* __restrict__ ohash, uint32_t* __restrict__ okey,
+               uint32_t* __restrict__ osorted, uint32_t* __restrict__ ostart) {
+  __shared__ __align__(16) uint32_t s_entry[kSmall];
+  __shared__ uint32_t s_sorted[kSmall];
+  const uint32_t i = threadIdx.x;  // (the block is n rounded up to whole warps)
+  uint32_t mine = 0xffffffffu;
+  if (i < n) {
+    const float3 p = make_float3(pred3[3 * i], pred3[3 * i + 1], pred3[3 * i + 2]);
+    const uint32_t h = hash_cell(cell_of(p.x, r), cell_of(p.y, r), cell_of(p.z, r));
+    const uint32_t key = fastmod(h, fm, n);
+    ohash[i] = h;
+    okey[i] = key;
+    ostart[i] = 0x7fffffffu;
+    mine = key << 16 | i;
+  }
+  s_entry[i] = mine;
+  __syncthreads();
+  uint32_t rank = 0;
+#pragma unroll 4
+  for (uint32_t k = 0; k < n; k += 4u) {
+    const uint4 e = *reinterpret_cast<const uint4*>(s_entry + k);
+    rank += (e.x < mine) + (e.y < mine) + (e.z < mine) + (e.w < mine);
+  }
+  if (i < n) s_sorted[rank] = mine;
+  __syncthreads();
+  if (i < n) {
+    const uint32_t e = s_sorted[i], key = e >> 16;
+    osorted[i] = e & 0xffffu;
+    if (i == 0u || s_sorted[i - 1u] >> 16 != key) ostart[key] = i;
+  }
+}
+
 }  // namespace
 
 }  // namespace sph
@@ -236,8 +277,12 @@ extern "C" int sph_spatial_lookup_static(const float* dpred3, uint32_t n,
     scratch = g_scratch_addr[dev];
   }
   const uint64_t fm = (~static_cast<uint64_t>(0)) / n + 1;
-  e = launch_pdl(false, k_lookup_static, kBlocks, kThreads, static_cast<cudaStream_t>(stream),
-                 dpred3, n, radius, fm, scratch, dhash, dkey, dsorted_ids, dstart);
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  e = n <= kSmall
+          ? launch_pdl(false, k_lookup_small, 1, static_cast<int>((n + 31u) / 32u * 32u), st,
+                       dpred3, n, radius, fm, dhash, dkey, dsorted_ids, dstart)
+          : launch_pdl(false, k_lookup_static, kBlocks, kThreads, st, dpred3, n, radius, fm,
+                       scratch, dhash, dkey, dsorted_ids, dstart);
   if (e != cudaSuccess)
     return fail(SPH_ERR_CUDA, std::string("lookup kernel: ") + cudaGetErrorString(e));
   return SPH_OK;
