@@ -2155,8 +2155,8 @@ auto visc_kernel(int gather, int lanes) {
 }
 
 // pick(gather), or the kernel of the next smaller batch that a block of `block`
-// threads has the registers for: 4 entries take up to 78 a thread, 8 up to 127,
-// where 1,024 threads leave 64 (two take 63 at most). 256 threads fit whatever
+// threads has the registers for: 4 entries take up to 77 a thread, 8 up to 127,
+// where 1,024 threads leave 64 (two take 62 at most). 256 threads fit whatever
 // a kernel takes and need no question. The results do not depend on the batch.
 template <class Pick> auto fitting_kernel(Pick pick, int gather, int block) {
   for (;;) {
